@@ -119,6 +119,35 @@ __device__ __forceinline__ void load_frame(const double* fg, size_t npad, size_t
     fr.t2 = {fg[6 * npad + f], fg[7 * npad + f], fg[8 * npad + f]};
 }
 
+// rho, velocity and u of a face's two states from its four stencil cells
+template <int NSP>
+__device__ __forceinline__ void interp_face(const L2R2<double>& r, bool lim, bool clip,
+                                            const Prim<double, NSP>& a, const Prim<double, NSP>& b,
+                                            const Prim<double, NSP>& c, const Prim<double, NSP>& d,
+                                            Prim<double, NSP>& Lf, Prim<double, NSP>& Rt) {
+    const double q[4][5] = {{a.vel.x, a.vel.y, a.vel.z, a.rho, a.u},
+                            {b.vel.x, b.vel.y, b.vel.z, b.rho, b.u},
+                            {c.vel.x, c.vel.y, c.vel.z, c.rho, c.u},
+                            {d.vel.x, d.vel.y, d.vel.z, d.rho, d.u}};
+    double L[5], R[5];
+    r.interp<5>(lim, clip, q, L, R);
+    Lf.vel = {L[0], L[1], L[2]}; Lf.rho = L[3]; Lf.u = L[4];
+    Rt.vel = {R[0], R[1], R[2]}; Rt.rho = R[3]; Rt.u = R[4];
+}
+// and the mass fractions
+template <int NSP>
+__device__ __forceinline__ void interp_massf(const L2R2<double>& r, bool lim, bool clip,
+                                             const Prim<double, NSP>& a, const Prim<double, NSP>& b,
+                                             const Prim<double, NSP>& c, const Prim<double, NSP>& d,
+                                             Prim<double, NSP>& Lf, Prim<double, NSP>& Rt) {
+    double q[4][NSP];
+#pragma unroll
+    for (int s = 0; s < NSP; ++s) {
+        q[0][s] = a.massf[s]; q[1][s] = b.massf[s]; q[2][s] = c.massf[s]; q[3][s] = d.massf[s];
+    }
+    r.interp<NSP>(lim, clip, q, Lf.massf, Rt.massf);
+}
+
 // update_thermo_from_rhou of a reconstructed state: ideal gas, or the
 // thermally perfect mixture started from the cell-centre temperature (the
 // state was copied from the cell, onedinterp.d / sfluidblock.d:2199-2208)
@@ -194,14 +223,9 @@ __global__ void k_flux(BlockView b, const SimDev* sim, FluxOpts o, int dir_arg) 
                 const double* len = b.cgeom + size_t(1 + dir) * b.npad;
                 L2R2<double> r;
                 r.prepare(len[cL1], len[cL0], len[cR0], len[cR1]);
-                r.scalar(o.limiter, o.clip, sL1.vel.x, sL0.vel.x, sR0.vel.x, sR1.vel.x, Lf.vel.x, Rt.vel.x);
-                r.scalar(o.limiter, o.clip, sL1.vel.y, sL0.vel.y, sR0.vel.y, sR1.vel.y, Lf.vel.y, Rt.vel.y);
-                r.scalar(o.limiter, o.clip, sL1.vel.z, sL0.vel.z, sR0.vel.z, sR1.vel.z, Lf.vel.z, Rt.vel.z);
+                interp_face<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                 if (NSP > 1) {
-#pragma unroll
-                    for (int q = 0; q < NSP; ++q)
-                        r.scalar(o.limiter, o.clip, sL1.massf[q], sL0.massf[q], sR0.massf[q],
-                                 sR1.massf[q], Lf.massf[q], Rt.massf[q]);
+                    interp_massf<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                     if (!scale_mass_fractions<double, NSP>(Lf.massf))
                         for (int q = 0; q < NSP; ++q) Lf.massf[q] = sL0.massf[q];
                     if (!scale_mass_fractions<double, NSP>(Rt.massf))
@@ -210,8 +234,6 @@ __global__ void k_flux(BlockView b, const SimDev* sim, FluxOpts o, int dir_arg) 
                     Lf.massf[0] = 1.0;
                     Rt.massf[0] = 1.0;
                 }
-                r.scalar(o.limiter, o.clip, sL1.rho, sL0.rho, sR0.rho, sR1.rho, Lf.rho, Rt.rho);
-                r.scalar(o.limiter, o.clip, sL1.u, sL0.u, sR0.u, sR1.u, Lf.u, Rt.u);
             }
             // codeForThermoUpdateBoth("rhou"), onedinterp.d:1039-1068: on failure
             // the cell-centre state (its velocity as above) is taken
@@ -564,14 +586,9 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
             {
                 L2R2<double> r;
                 r.prepare(wl[0], wl[1], wl[2], wl[3]);
-                r.scalar(o.limiter, o.clip, sL1.vel.x, sL0.vel.x, sR0.vel.x, sR1.vel.x, Lf.vel.x, Rt.vel.x);
-                r.scalar(o.limiter, o.clip, sL1.vel.y, sL0.vel.y, sR0.vel.y, sR1.vel.y, Lf.vel.y, Rt.vel.y);
-                r.scalar(o.limiter, o.clip, sL1.vel.z, sL0.vel.z, sR0.vel.z, sR1.vel.z, Lf.vel.z, Rt.vel.z);
+                interp_face<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                 if (NSP > 1) {
-#pragma unroll
-                    for (int q = 0; q < NSP; ++q)
-                        r.scalar(o.limiter, o.clip, sL1.massf[q], sL0.massf[q], sR0.massf[q],
-                                 sR1.massf[q], Lf.massf[q], Rt.massf[q]);
+                    interp_massf<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                     if (!scale_mass_fractions<double, NSP>(Lf.massf))
                         for (int q = 0; q < NSP; ++q) Lf.massf[q] = sL0.massf[q];
                     if (!scale_mass_fractions<double, NSP>(Rt.massf))
@@ -580,8 +597,6 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
                     Lf.massf[0] = 1.0;
                     Rt.massf[0] = 1.0;
                 }
-                r.scalar(o.limiter, o.clip, sL1.rho, sL0.rho, sR0.rho, sR1.rho, Lf.rho, Rt.rho);
-                r.scalar(o.limiter, o.clip, sL1.u, sL0.u, sR0.u, sR1.u, Lf.u, Rt.u);
             }
             // codeForThermoUpdateBoth("rhou"), onedinterp.d:1039-1068: on failure
             // the cell-centre state (its velocity in the face frame) is taken
@@ -667,7 +682,7 @@ __global__ void k_update(BlockView b, SimDev* sim, GasConsts gas, int stage, int
                 integral[v] -= F[v * b.npad + fq[q]] * area;
             }
         }
-        double vol_inv = 1.0 / b.cgeom[c];
+        double vol_inv = fdiv(1.0, b.cgeom[c]);
         double Un[NV];
         if (stage == 1) {
 #pragma unroll
@@ -693,7 +708,7 @@ __global__ void k_update(BlockView b, SimDev* sim, GasConsts gas, int stage, int
             set_status(sim, -5);
             data_bad = true;
         } else {
-            double dinv = 1.0 / rho;
+            double dinv = fdiv(1.0, rho);
             vx = Un[1] * dinv; vy = Un[2] * dinv; vz = Un[3] * dinv;
             u = Un[4] * dinv;
             double ke = 0.5 * (vx * vx + vy * vy + vz * vz);

@@ -191,7 +191,7 @@ __device__ __forceinline__ void cell_pressure(Prim<R, 1>& s, const GasConsts& ga
 //
 // vaL, vaR (optional, with the limiter on): the van Albada values of the
 // cells L0 and R0 for this direction, at stride vs, in the order rho, vx, vy,
-// vz, u of the global frame (L2R2::va).
+// vz, u of the global frame (L2R2::va_terms).
 template <typename R, int FLUX, int DIR>
 __device__ __forceinline__ void face_flux(Prim<R, 1> sL1, Prim<R, 1> sL0, Prim<R, 1> sR0,
                                           Prim<R, 1> sR1, const L2R2<R>& w, const FluxOpts& o,
@@ -216,20 +216,20 @@ __device__ __forceinline__ void face_flux(Prim<R, 1> sL1, Prim<R, 1> sL0, Prim<R
                           sR1.vel.y, Lf.vel.y, Rt.vel.y);
             w.scalar_with(vaL[c2 * vs], vaR[c2 * vs], clip, sL1.vel.z, sL0.vel.z, sR0.vel.z,
                           sR1.vel.z, Lf.vel.z, Rt.vel.z);
-        } else {
-            w.scalar(lim, clip, sL1.vel.x, sL0.vel.x, sR0.vel.x, sR1.vel.x, Lf.vel.x, Rt.vel.x);
-            w.scalar(lim, clip, sL1.vel.y, sL0.vel.y, sR0.vel.y, sR1.vel.y, Lf.vel.y, Rt.vel.y);
-            w.scalar(lim, clip, sL1.vel.z, sL0.vel.z, sR0.vel.z, sR1.vel.z, Lf.vel.z, Rt.vel.z);
-        }
-        Lf.massf[0] = R(1.0);
-        Rt.massf[0] = R(1.0);
-        if (vaL) {
             w.scalar_with(vaL[0], vaR[0], clip, sL1.rho, sL0.rho, sR0.rho, sR1.rho, Lf.rho, Rt.rho);
             w.scalar_with(vaL[4 * vs], vaR[4 * vs], clip, sL1.u, sL0.u, sR0.u, sR1.u, Lf.u, Rt.u);
         } else {
-            w.scalar(lim, clip, sL1.rho, sL0.rho, sR0.rho, sR1.rho, Lf.rho, Rt.rho);
-            w.scalar(lim, clip, sL1.u, sL0.u, sR0.u, sR1.u, Lf.u, Rt.u);
+            const R q[4][5] = {{sL1.vel.x, sL1.vel.y, sL1.vel.z, sL1.rho, sL1.u},
+                               {sL0.vel.x, sL0.vel.y, sL0.vel.z, sL0.rho, sL0.u},
+                               {sR0.vel.x, sR0.vel.y, sR0.vel.z, sR0.rho, sR0.u},
+                               {sR1.vel.x, sR1.vel.y, sR1.vel.z, sR1.rho, sR1.u}};
+            R l[5], r[5];
+            w.template interp<5>(lim, clip, q, l, r);
+            Lf.vel = {l[0], l[1], l[2]}; Lf.rho = l[3]; Lf.u = l[4];
+            Rt.vel = {r[0], r[1], r[2]}; Rt.rho = r[3]; Rt.u = r[4];
         }
+        Lf.massf[0] = R(1.0);
+        Rt.massf[0] = R(1.0);
         R T;
         if (!ideal_rhou<R>(o.gas, Lf.rho, Lf.u, Lf.p, T)) { Lf = sL0; cell_pressure(Lf, o.gas); }
         if (!ideal_rhou<R>(o.gas, Rt.rho, Rt.u, Rt.p, T)) { Rt = sR0; cell_pressure(Rt, o.gas); }
@@ -554,11 +554,15 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
                         off = (cj + 1) * PI + (ci + 2);
                         step = PI; dir = 1; dst = VAj + g; vs = S::NVJ;
                     }
+                    R nu[5], de[5], va[5];
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
                         const R* q = pk + f * FS + off;
-                        dst[f * vs] = w[dir].va(q[-step], q[0], q[step]);
+                        w[dir].va_terms(q[-step], q[0], q[step], nu[f], de[f]);
                     }
+                    fdiv_va<5>(nu, de, va);
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) dst[f * vs] = va[f];
                 }
             }
             // plane k+2 and the limiter values of plane k are in place (plane k
@@ -646,7 +650,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
                     s -= double(Fbot[v]) * (-1.0 * aT);
                     integral[v] = s;
                 }
-                const double vol_inv = 1.0 / d.vol;
+                const double vol_inv = fdiv(1.0, d.vol);
                 const size_t c = (size_t(k) * d.nj + j) * d.ni + i;
                 double Un[5];
                 if (stage == 1) {
@@ -670,7 +674,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
                     if (atomicCAS(&sim->status, 0, -5) == 0) sim->status_step = sim->step;
                     ok = false;
                 } else {
-                    const double dinv = 1.0 / rho;
+                    const double dinv = fdiv(1.0, rho);
                     vx = Un[1] * dinv; vy = Un[2] * dinv; vz = Un[3] * dinv;
                     u = Un[4] * dinv;
                     const double ke = 0.5 * (vx * vx + vy * vy + vz * vz);
