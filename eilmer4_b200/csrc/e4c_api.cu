@@ -125,7 +125,8 @@ void Ctx::enqueue_stage(const std::vector<int>& hs, int stage, int final_stage) 
     launch_as(*this, E4C_KCLASS_OTHER, 1, [&] { launch_reset_bad(d_sim, stream); });
     bool any_fused = false;
     for (int h : hs) any_fused = any_fused || blocks[h].fused;
-    if (any_fused) launch_as(*this, E4C_KCLASS_STAGE, 1, [&] { fused_stage_all(stage); });
+    if (any_fused)
+        launch_as(*this, E4C_KCLASS_STAGE, fused_stage_kernels(), [&] { fused_stage_all(stage); });
     for (int h : hs) {
         const BlockHost& b = blocks[h];
         if (!b.fused) launch_as(*this, E4C_KCLASS_BC, 1, [&] { launch_bc(b.v, d_sim, stream); });
@@ -972,7 +973,8 @@ int e4c_profile_steps(int nsteps, double* ms, int* launches) {
 static int read_sim(SimDev& s);
 
 static bool tile_available(int ti, int tj) {
-    const int tiles[][2] = {{32, 8}, {32, 4}, {16, 8}, {64, 4}, {16, 16}, {32, 16}};
+    const int tiles[][2] = {{32, 8}, {32, 4}, {16, 8}, {64, 4},
+                            {16, 16}, {32, 16}, {32, 14}};
     for (auto& t : tiles)
         if (t[0] == ti && t[1] == tj) return true;
     return false;
@@ -1058,7 +1060,8 @@ int e4c_autotune(int nsteps, int* ti, int* tj, int* kc, double* ms_per_step) {
             cudaMemcpyAsync(const_cast<void*>(x.src), x.dst, x.bytes, cudaMemcpyDeviceToDevice,
                             c.stream);
     };
-    const int tiles[][2] = {{32, 8}, {32, 4}, {16, 8}, {64, 4}, {16, 16}, {32, 16}};
+    const int tiles[][2] = {{32, 8}, {32, 4}, {16, 8}, {64, 4},
+                            {16, 16}, {32, 16}, {32, 14}};
     const int kcs[] = {16, 32, 64, 128};
     int best_ti = c.tile_ti, best_tj = c.tile_tj, best_kc = c.tile_kc;
     double best = 1.0e300;

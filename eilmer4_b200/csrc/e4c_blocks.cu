@@ -329,9 +329,16 @@ int Ctx::prepare_fused() {
 }
 
 void Ctx::fused_stage_all(int stage) {
-    FusedLaunch L{d_descs, nfused, fused_items, tile_kc, tile_ti, tile_tj, fused_grid, d_item_order};
+    FusedLaunch L{d_descs, nfused, fused_items, tile_kc, tile_ti, tile_tj, fused_grid, d_item_order,
+                  max_cells_fused};
     if (cfg.precision == E4C_PREC_FP32_FLUX) f32::fused_stage(L, d_sim, gas, fopts, stage, stream);
     else f64::fused_stage(L, d_sim, gas, fopts, stage, stream);
+}
+
+int Ctx::fused_stage_kernels() const {
+    return cfg.precision == E4C_PREC_FP32_FLUX
+               ? f32::fused_kernels(cfg.flux_calculator, tile_ti, tile_tj)
+               : f64::fused_kernels(cfg.flux_calculator, tile_ti, tile_tj);
 }
 
 void Ctx::fused_dt_all(SimDev* sim, const double* dt_current) {

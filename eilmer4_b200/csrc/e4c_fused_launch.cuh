@@ -8,6 +8,9 @@
 #if E4C_FUSED_WS
 #include "e4c_fused_ws.cuh"
 #endif
+#if E4C_FUSED_WS64
+#include "e4c_fused_ws64.cuh"
+#endif
 
 #ifndef E4C_FUSED_R
 #error "define E4C_FUSED_R (double or float) before including this file"
@@ -77,11 +80,58 @@ static int occupancy_ws() {
     return n;
 }
 
-#define E4C_WS_TILES(X) X(4) X(8) X(16)
+#define E4C_WS_TILES(X) X(4) X(8) X(14) X(16)
+#endif
+
+#if E4C_FUSED_WS64
+// 32-wide tiles of the FP64 form: the kernel with edge warps and per-cell
+// reconstruction, the adaptive flux's shock points detected in a pass before it
+template <int FLUX, int TJ>
+static int launch_ws64(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, const FluxOpts& o,
+                       int stage, cudaStream_t s) {
+    constexpr size_t smem = ws64::Lay<TJ>::bytes;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaFuncSetAttribute(ws64::k_fused_stage_ws64<FLUX, TJ>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        attr_set = true;
+    }
+    const FusedDesc* descs = static_cast<const FusedDesc*>(L.descs);
+    if (FLUX == 3) {
+        int gx = (L.max_cells + 255) / 256;
+        if (gx > 148 * 16) gx = 148 * 16;
+        ws64::k_fused_shock<<<dim3(gx, L.nblocks), 256, 0, s>>>(descs, sim, gas,
+                                                                o.compression_tol, stage);
+    }
+    ws64::k_fused_stage_ws64<FLUX, TJ><<<L.grid, ws64::Lay<TJ>::threads, smem, s>>>(
+        descs, L.nblocks, L.nitems, L.kc, sim, gas, o, stage, L.order);
+    return 0;
+}
+
+template <int FLUX, int TJ>
+static int occupancy_ws64() {
+    constexpr size_t smem = ws64::Lay<TJ>::bytes;
+    cudaFuncSetAttribute(ws64::k_fused_stage_ws64<FLUX, TJ>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ws64::k_fused_stage_ws64<FLUX, TJ>,
+                                                      ws64::Lay<TJ>::threads, smem) != cudaSuccess)
+        return 0;
+    return n;
+}
+
+#define E4C_WS64_TILES(X) X(4) X(8) X(14)
 #endif
 
 // Tile shapes available to the autotuner: (TI, TJ).
-#define E4C_TILES(X) X(32, 8) X(32, 4) X(16, 8) X(64, 4) X(16, 16) X(32, 16)
+// The per-face kernel serves the shapes the kernels above do not: 16- and
+// 64-wide tiles, 32x16 in FP64 (the row kernel's shared memory stops at 14
+// rows), and 32-wide ones of the FP32-flux form for first-order reconstruction.
+#if E4C_FUSED_WS64
+#define E4C_TILES(X) X(16, 8) X(64, 4) X(16, 16) X(32, 16)
+#else
+#define E4C_TILES(X) X(32, 8) X(32, 4) X(16, 8) X(64, 4) X(16, 16) X(32, 16) X(32, 14)
+#endif
 
 int fused_stage(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, const FluxOpts& o,
                 int stage, cudaStream_t s) {
@@ -94,6 +144,19 @@ int fused_stage(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, const F
         }
         E4C_WS_TILES(E4C_WS_CASE)
 #undef E4C_WS_CASE
+    }
+#endif
+#if E4C_FUSED_WS64
+    if (L.ti == 32) {
+#define E4C_WS64_CASE(TJ_)                                                          \
+        if (L.tj == TJ_) {                                                          \
+            if (o.flux == 1) return launch_ws64<1, TJ_>(L, sim, gas, o, stage, s);  \
+            if (o.flux == 2) return launch_ws64<2, TJ_>(L, sim, gas, o, stage, s);  \
+            if (o.flux == 3) return launch_ws64<3, TJ_>(L, sim, gas, o, stage, s);  \
+            return launch_ws64<0, TJ_>(L, sim, gas, o, stage, s);                   \
+        }
+        E4C_WS64_TILES(E4C_WS64_CASE)
+#undef E4C_WS64_CASE
     }
 #endif
 // Hanel and the adaptive Hanel/AUSMDV flux: the FP64 form only
@@ -120,6 +183,19 @@ int fused_occupancy(int flux, int ti, int tj) {
 #undef E4C_WS_CASE
     }
 #endif
+#if E4C_FUSED_WS64
+    if (ti == 32) {
+#define E4C_WS64_CASE(TJ_)                                                          \
+        if (tj == TJ_) {                                                            \
+            if (flux == 1) return occupancy_ws64<1, TJ_>();                         \
+            if (flux == 2) return occupancy_ws64<2, TJ_>();                         \
+            if (flux == 3) return occupancy_ws64<3, TJ_>();                         \
+            return occupancy_ws64<0, TJ_>();                                        \
+        }
+        E4C_WS64_TILES(E4C_WS64_CASE)
+#undef E4C_WS64_CASE
+    }
+#endif
 #define E4C_CASE(TI_, TJ_)                                          \
     if (ti == TI_ && tj == TJ_) {                                  \
         if constexpr (sizeof(RT) == 8) {                           \
@@ -131,6 +207,20 @@ int fused_occupancy(int flux, int ti, int tj) {
     E4C_TILES(E4C_CASE)
 #undef E4C_CASE
     return 0;
+}
+
+// kernels that one fused_stage call launches
+int fused_kernels(int flux, int ti, int tj) {
+#if E4C_FUSED_WS64
+    if (flux == 3 && ti == 32) {
+#define E4C_WS64_CASE(TJ_) \
+        if (tj == TJ_) return 2;
+        E4C_WS64_TILES(E4C_WS64_CASE)
+#undef E4C_WS64_CASE
+    }
+#endif
+    (void)flux; (void)ti; (void)tj;
+    return 1;
 }
 
 void fused_dt(const void* descs, int nfused, int gx, SimDev* sim, const GasConsts& gas,

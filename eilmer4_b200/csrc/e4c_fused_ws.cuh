@@ -59,16 +59,21 @@ struct Lay {
     static constexpr int o_a = o_qjm + 5 * QJ;
     static constexpr int o_fi = o_a + AN;
     static constexpr int o_fj = o_fi + 5 * FI;
-    static constexpr int words = o_fj + 5 * FJ;
+    static constexpr int o_plan = o_fj + 5 * FJ;  // plan_tile's table (ints)
+    static constexpr int words = o_plan + PLANE;
     static constexpr size_t bytes = sizeof(float) * size_t(words);
     static constexpr int threads = 32 * (TJ + NEW);
     static constexpr int min_blocks =
         (E4C_WS_WARPS / (TJ + NEW)) > 0 ? E4C_WS_WARPS / (TJ + NEW) : 1;
 };
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+__device__ __forceinline__ void cp_async_elem(float* dst, const float* src) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_elem(double* dst, const double* src) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -145,101 +150,241 @@ __device__ __forceinline__ float sound_speed(float u, const GasConsts& g) {
     return sqrtf(float(g.gamma) * float(g.Rgas) * (u * float(g.Cvinv)));
 }
 
-// Edge threads: queue the copies of halo plane kk of a tile into ring slot
-// `slot` (5 fields), the ghost cells made from the boundary conditions as
-// load_plane makes them.  Inflow ghosts are stored at once; every other cell
-// is copied from its source with cp.async.  Returns, two bits per position
-// this thread handles, the velocity component a slip wall negates once the
-// copies have landed (fixup_plane).
-template <int TJ>
+// Queue the copies of ring position e of halo plane kk of a tile into `slot`
+// (5 fields), a ghost cell made from its boundary condition as load_plane makes
+// it.  Inflow ghosts are stored at once; every other cell is copied from its
+// source with cp.async.  Returns the velocity component a slip wall negates
+// once the copies have landed (1..3), or 0.
+template <int TJ, typename R>
+__device__ __forceinline__ unsigned queue_cell(const FusedDesc* __restrict__ descs, int stage,
+                                               const FusedDesc& d, const R* __restrict__ W,
+                                               R* slot, int i0, int j0, int kk, int e) {
+    constexpr int NPOS = PI * (TJ + 4);
+    unsigned fix = 0u;
+    const int x = e % PI, r = e / PI;
+    int gi = i0 - 2 + x, gj = j0 - 2 + r, gk = kk;
+    const bool oi = gi < 0 || gi >= d.ni;
+    const bool oj = gj < 0 || gj >= d.nj;
+    const bool ok = gk < 0 || gk >= d.nk;
+    if (int(oi) + int(oj) + int(ok) > 1) return 0u;
+    int which = -1, layer = 0;
+    if (oi) {
+        if (gi < 0) { which = WEST; layer = -gi - 1; }
+        else { which = EAST; layer = gi - d.ni; }
+    } else if (oj) {
+        if (gj < 0) { which = SOUTH; layer = -gj - 1; }
+        else { which = NORTH; layer = gj - d.nj; }
+    } else if (ok) {
+        if (gk < 0) { which = BOTTOM; layer = -gk - 1; }
+        else { which = TOP; layer = gk - d.nk; }
+    }
+    if (layer > 1) return 0u;
+    const int type = which >= 0 ? d.bc[which] : -1;
+    if (type == 1) {  // supersonic inflow: both ghost layers hold the inflow state
+#pragma unroll
+        for (int f = 0; f < 5; ++f) slot[f * NPOS + e] = R(d.inflow[f]);
+        return 0u;
+    }
+    const R* src;
+    size_t c, snc;
+    if (type == 3) {  // full-face copy from the partner block (opposite faces)
+        const FusedDesc& o = descs[d.ex[which]];
+        int si = gi, sj = gj, sk = gk;
+        switch (which) {
+            case WEST: si = o.ni - 1 - layer; break;
+            case EAST: si = layer; break;
+            case SOUTH: sj = o.nj - 1 - layer; break;
+            case NORTH: sj = layer; break;
+            case BOTTOM: sk = o.nk - 1 - layer; break;
+            default: sk = layer; break;
+        }
+        snc = size_t(o.ni) * o.nj * o.nk;
+        c = (size_t(sk) * o.nj + sj) * o.ni + si;
+        src = static_cast<const R*>(stage == 1 ? o.WA : o.WB);
+    } else {
+        if (which >= 0) {
+            // the mirror cell for a slip wall, the first interior cell for
+            // the zero-order extrapolation outflow
+            const int s = (type == 2) ? 0 : layer;
+            switch (which) {
+                case WEST: gi = s; break;
+                case EAST: gi = d.ni - 1 - s; break;
+                case SOUTH: gj = s; break;
+                case NORTH: gj = d.nj - 1 - s; break;
+                case BOTTOM: gk = s; break;
+                default: gk = d.nk - 1 - s; break;
+            }
+            // reflect_normal_velocity with an axis frame
+            if (type == 0)
+                fix = (which == WEST || which == EAST) ? 1u
+                      : (which == SOUTH || which == NORTH) ? 2u : 3u;
+        }
+        snc = size_t(d.ni) * d.nj * d.nk;
+        c = (size_t(gk) * d.nj + gj) * d.ni + gi;
+        src = W;
+    }
+#pragma unroll
+    for (int f = 0; f < 5; ++f) cp_async_elem(slot + f * NPOS + e, src + f * snc + c);
+    return fix;
+}
+
+// Edge threads: halo plane kk of a tile into ring slot `slot`, position by
+// position; returns two bits per position this thread handles (fixup_plane).
+template <int TJ, typename R>
 __device__ __forceinline__ unsigned queue_plane(const FusedDesc* __restrict__ descs, int stage,
-                                                const FusedDesc& d, const float* __restrict__ W,
-                                                float* slot, int i0, int j0, int kk, int et) {
-    constexpr int NPOS = Lay<TJ>::PLANE;
-    const size_t nc = size_t(d.ni) * d.nj * d.nk;
+                                                const FusedDesc& d, const R* __restrict__ W,
+                                                R* slot, int i0, int j0, int kk, int et) {
+    constexpr int NPOS = PI * (TJ + 4);
+    unsigned fix = 0u;
+    int m = 0;
+    for (int e = et; e < NPOS; e += NE, ++m)
+        fix |= queue_cell<TJ>(descs, stage, d, W, slot, i0, j0, kk, e) << (2 * m);
+    return fix;
+}
+
+// The plan of a tile's planes inside the block (0 <= kk < nk), the same for
+// every one of them: per ring position the source cell's offset in its plane
+// and which array it lies in (PlanSrc: the block's own, or the partner's across
+// one of its four i and j faces), -1 for a position that is never copied
+// (unread, or beyond an inflow face: those are stored into all four slots here,
+// nothing overwrites them), -2 for one that queue_cell serves.  Made once per
+// work item by the edge threads, each its own positions (so no barrier);
+// returns their fixup bits.  It leaves a plane's queueing to one shared-memory
+// load and five copies per position (measured with the FP64 kernel: deciding
+// every position anew made the edge warps the longer side of the plane's first
+// phase, and a third of all stall cycles were waits for them at its barrier).
+template <typename R>
+struct PlanSrc {
+    const R* W;       // first cell of plane 0
+    size_t nc;        // field stride
+    size_t plane;     // plane stride
+};
+constexpr int kPlanBits = 28;   // offset bits; the source's number above them
+
+// the five sources of a block, by one thread (read after a barrier)
+template <typename R>
+__device__ __forceinline__ void plan_sources(const FusedDesc* __restrict__ descs, int stage,
+                                             const FusedDesc& d, const R* W, PlanSrc<R>* src) {
+    src[0] = PlanSrc<R>{W, size_t(d.ni) * d.nj * d.nk, size_t(d.ni) * d.nj};
+    const int faces[4] = {WEST, EAST, SOUTH, NORTH};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (d.bc[faces[q]] == 3) {
+            const FusedDesc& o = descs[d.ex[faces[q]]];
+            src[1 + q] = PlanSrc<R>{static_cast<const R*>(stage == 1 ? o.WA : o.WB),
+                                    size_t(o.ni) * o.nj * o.nk, size_t(o.ni) * o.nj};
+        }
+    }
+}
+
+template <int TJ, typename R>
+__device__ __forceinline__ unsigned plan_tile(const FusedDesc* __restrict__ descs,
+                                              const FusedDesc& d, int* plan, R* ring, int i0,
+                                              int j0, int et) {
+    constexpr int NPOS = PI * (TJ + 4);
     unsigned fix = 0u;
     int m = 0;
     for (int e = et; e < NPOS; e += NE, ++m) {
         const int x = e % PI, r = e / PI;
-        int gi = i0 - 2 + x, gj = j0 - 2 + r, gk = kk;
+        int gi = i0 - 2 + x, gj = j0 - 2 + r;
         const bool oi = gi < 0 || gi >= d.ni;
         const bool oj = gj < 0 || gj >= d.nj;
-        const bool ok = gk < 0 || gk >= d.nk;
-        if (int(oi) + int(oj) + int(ok) > 1) continue;
-        int which = -1, layer = 0;
-        if (oi) {
-            if (gi < 0) { which = WEST; layer = -gi - 1; }
-            else { which = EAST; layer = gi - d.ni; }
-        } else if (oj) {
-            if (gj < 0) { which = SOUTH; layer = -gj - 1; }
-            else { which = NORTH; layer = gj - d.nj; }
-        } else if (ok) {
-            if (gk < 0) { which = BOTTOM; layer = -gk - 1; }
-            else { which = TOP; layer = gk - d.nk; }
-        }
-        if (layer > 1) continue;
-        const int type = which >= 0 ? d.bc[which] : -1;
-        if (type == 1) {  // supersonic inflow: both ghost layers hold the inflow state
+        int off = -1;
+        if (!(oi && oj)) {
+            int which = -1, layer = 0, code = 0;
+            if (oi) {
+                if (gi < 0) { which = WEST; layer = -gi - 1; code = 1; }
+                else { which = EAST; layer = gi - d.ni; code = 2; }
+            } else if (oj) {
+                if (gj < 0) { which = SOUTH; layer = -gj - 1; code = 3; }
+                else { which = NORTH; layer = gj - d.nj; code = 4; }
+            }
+            const int type = which >= 0 ? d.bc[which] : -1;
+            if (layer <= 1) {
+                int pitch = d.ni;
+                if (type == 3) {
+                    const FusedDesc& o = descs[d.ex[which]];
+                    switch (which) {
+                        case WEST: gi = o.ni - 1 - layer; break;
+                        case EAST: gi = layer; break;
+                        case SOUTH: gj = o.nj - 1 - layer; break;
+                        default: gj = layer; break;
+                    }
+                    pitch = o.ni;
+                } else {
+                    code = 0;
+                    if (type == 1) {
 #pragma unroll
-            for (int f = 0; f < 5; ++f) slot[f * NPOS + e] = float(d.inflow[f]);
+                        for (int q = 0; q < 20; ++q)
+                            ring[q * NPOS + e] = R(d.inflow[q % 5]);
+                    } else if (which >= 0) {
+                        const int s = (type == 2) ? 0 : layer;
+                        switch (which) {
+                            case WEST: gi = s; break;
+                            case EAST: gi = d.ni - 1 - s; break;
+                            case SOUTH: gj = s; break;
+                            default: gj = d.nj - 1 - s; break;
+                        }
+                        if (type == 0)
+                            fix |= ((which == WEST || which == EAST) ? 1u : 2u) << (2 * m);
+                    }
+                }
+                if (type != 1) {
+                    const long long o = (long long)gj * pitch + gi;
+                    off = o < (1ll << kPlanBits) ? int(o) | (code << kPlanBits) : -2;
+                    if (off == -2) fix &= ~(3u << (2 * m));
+                }
+            }
+        }
+        plan[e] = off;
+    }
+    return fix;
+}
+
+// queue_plane by the tile's plan; planes beyond the block's k faces go
+// position by position.
+template <int TJ, typename R>
+__device__ __forceinline__ unsigned queue_planned(const FusedDesc* __restrict__ descs, int stage,
+                                                  const FusedDesc& d, const R* __restrict__ W,
+                                                  R* slot, int i0, int j0, int kk, int et,
+                                                  const int* plan, const PlanSrc<R>* srcs,
+                                                  unsigned plan_fix) {
+    constexpr int NPOS = PI * (TJ + 4);
+    if (kk < 0 || kk >= d.nk) return queue_plane<TJ>(descs, stage, d, W, slot, i0, j0, kk, et);
+    const PlanSrc<R> own = srcs[0];
+    const R* Wk = own.W + size_t(kk) * own.plane;
+    unsigned fix = plan_fix;
+    int m = 0;
+    for (int e = et; e < NPOS; e += NE, ++m) {
+        const int off = plan[e];
+        if (off < 0) {
+            if (off == -2)
+                fix |= queue_cell<TJ>(descs, stage, d, W, slot, i0, j0, kk, e) << (2 * m);
             continue;
         }
-        const float* src;
-        size_t c, snc;
-        if (type == 3) {  // full-face copy from the partner block (opposite faces)
-            const FusedDesc& o = descs[d.ex[which]];
-            int si = gi, sj = gj, sk = gk;
-            switch (which) {
-                case WEST: si = o.ni - 1 - layer; break;
-                case EAST: si = layer; break;
-                case SOUTH: sj = o.nj - 1 - layer; break;
-                case NORTH: sj = layer; break;
-                case BOTTOM: sk = o.nk - 1 - layer; break;
-                default: sk = layer; break;
-            }
-            snc = size_t(o.ni) * o.nj * o.nk;
-            c = (size_t(sk) * o.nj + sj) * o.ni + si;
-            src = static_cast<const float*>(stage == 1 ? o.WA : o.WB);
-        } else {
-            if (which >= 0) {
-                // the mirror cell for a slip wall, the first interior cell for
-                // the zero-order extrapolation outflow
-                const int s = (type == 2) ? 0 : layer;
-                switch (which) {
-                    case WEST: gi = s; break;
-                    case EAST: gi = d.ni - 1 - s; break;
-                    case SOUTH: gj = s; break;
-                    case NORTH: gj = d.nj - 1 - s; break;
-                    case BOTTOM: gk = s; break;
-                    default: gk = d.nk - 1 - s; break;
-                }
-                if (type == 0) {
-                    // reflect_normal_velocity with an axis frame
-                    const unsigned comp = (which == WEST || which == EAST) ? 1u
-                                          : (which == SOUTH || which == NORTH) ? 2u : 3u;
-                    fix |= comp << (2 * m);
-                }
-            }
-            snc = nc;
-            c = (size_t(gk) * d.nj + gj) * d.ni + gi;
-            src = W;
+        const R* src = Wk + off;
+        size_t nc = own.nc;
+        if (off >> kPlanBits) {
+            const PlanSrc<R> p = srcs[off >> kPlanBits];
+            src = p.W + size_t(kk) * p.plane + (off & ((1 << kPlanBits) - 1));
+            nc = p.nc;
         }
 #pragma unroll
-        for (int f = 0; f < 5; ++f) cp_async4(slot + f * NPOS + e, src + f * snc + c);
+        for (int f = 0; f < 5; ++f) cp_async_elem(slot + f * NPOS + e, src + f * nc);
     }
     return fix;
 }
 
 // After cp_async_wait_all: negate the normal velocity of this thread's
 // slip-wall ghost cells.
-template <int TJ>
-__device__ __forceinline__ void fixup_plane(float* slot, unsigned fix, int et) {
-    constexpr int NPOS = Lay<TJ>::PLANE;
+template <int TJ, typename R>
+__device__ __forceinline__ void fixup_plane(R* slot, unsigned fix, int et) {
+    constexpr int NPOS = PI * (TJ + 4);
     int m = 0;
     for (int e = et; e < NPOS && fix; e += NE, ++m) {
         const unsigned comp = (fix >> (2 * m)) & 3u;
         if (comp) {
-            float* p = slot + comp * NPOS + e;
+            R* p = slot + comp * NPOS + e;
             *p = -*p;
             fix &= ~(3u << (2 * m));
         }
@@ -271,6 +416,8 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
     float* As = sm + L::o_a;
     float* Fi = sm + L::o_fi;
     float* Fj = sm + L::o_fj;
+    int* plan = reinterpret_cast<int*>(sm + L::o_plan);
+    __shared__ PlanSrc<float> s_src[5];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool edge = warp >= TJ;
     const int et = threadIdx.x - 32 * TJ;   // edge thread index (edge warps)
@@ -308,13 +455,17 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
 #pragma unroll
         for (int q = 0; q < 3; ++q) w[q] = float(1.0e-12 * d.len[q] * d.len[q]);
 
+        if (threadIdx.x == 0) plan_sources<float>(descs, stage, d, Win, s_src);
+        __syncthreads();
         // prologue: planes k0-2 .. k0+1
+        unsigned plan_fix = 0u;
         if (edge) {
+            plan_fix = plan_tile<TJ>(descs, d, plan, ring, i0, j0, et);
             unsigned fx[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                fx[q] = queue_plane<TJ>(descs, stage, d, Win, slot_of(k0 - 2 + q), i0, j0,
-                                        k0 - 2 + q, et);
+                fx[q] = queue_planned<TJ>(descs, stage, d, Win, slot_of(k0 - 2 + q), i0, j0,
+                                          k0 - 2 + q, et, plan, s_src, plan_fix);
             cp_async_wait_all();
 #pragma unroll
             for (int q = 0; q < 4; ++q) fixup_plane<TJ>(slot_of(k0 - 2 + q), fx[q], et);
@@ -350,7 +501,8 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
         __syncthreads();   // plane k0-2's slot takes plane k0+2 next
         if (edge) {
             float* s = slot_of(k0 + 2);
-            const unsigned fx = queue_plane<TJ>(descs, stage, d, Win, s, i0, j0, k0 + 2, et);
+            const unsigned fx = queue_planned<TJ>(descs, stage, d, Win, s, i0, j0, k0 + 2, et, plan,
+                                                  s_src, plan_fix);
             cp_async_wait_all();
             fixup_plane<TJ>(s, fx, et);
         }
@@ -365,8 +517,8 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
             // ---- phase A: reconstruction ------------------------------------------
             if (edge) {
                 if (load_next)
-                    fx_next = queue_plane<TJ>(descs, stage, d, Win, slot_of(k + 3), i0, j0, k + 3,
-                                              et);
+                    fx_next = queue_planned<TJ>(descs, stage, d, Win, slot_of(k + 3), i0, j0, k + 3,
+                                                et, plan, s_src, plan_fix);
                 // halo cells: rows -1 and TJ (j-direction), columns -1 and 32
                 // (i-direction), with their sound speed
                 for (int t = et; t < 64 + 2 * TJ; t += NE) {

@@ -169,6 +169,7 @@ struct Ctx {
     std::vector<int> all_blocks() const;
     // fused uniform path
     void fused_stage_all(int stage);
+    int fused_stage_kernels() const;   // kernels of one fused_stage_all
     void fused_dt_all(SimDev* sim, const double* dt_current);
     int fused_upload(BlockHost& b, const double* prim);
     int fused_upload_cons(BlockHost& b, const double* cons);

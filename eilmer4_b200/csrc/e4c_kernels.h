@@ -96,6 +96,7 @@ struct FusedLaunch {
     int ti, tj;             // tile shape
     int grid;               // persistent CTAs
     const int* order;       // work items, costliest first (device array of nitems)
+    int max_cells;          // cells of the largest block
 };
 
 #define E4C_DECLARE_FUSED(NS)                                                                \
@@ -103,6 +104,7 @@ struct FusedLaunch {
     int fused_stage(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, const FluxOpts& o, \
                     int stage, cudaStream_t s);                                              \
     int fused_occupancy(int flux, int ti, int tj);                                           \
+    int fused_kernels(int flux, int ti, int tj);                                             \
     void fused_dt(const void* descs, int nfused, int gx, SimDev* sim, const GasConsts& gas,  \
                   double cfl_value, const double* dt_current, cudaStream_t s);              \
     void fused_dt_one(const FusedDesc& d, unsigned long long* acc, int gx,                   \
