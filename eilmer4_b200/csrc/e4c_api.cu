@@ -328,6 +328,7 @@ int e4c_init(const e4c_config* cfg) {
     c.fopts.compression_tol = cfg->compression_tolerance;
     c.fopts.row_run_i = 0;
     c.fopts.row_run_jk = 0;
+    c.tile_auto = true;
     E4C_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     E4C_CUDA(cudaStreamCreateWithFlags(&c.h2d_stream, cudaStreamNonBlocking));
     E4C_CUDA(cudaStreamCreateWithFlags(&c.d2h_stream, cudaStreamNonBlocking));
@@ -984,6 +985,7 @@ int e4c_set_tile(int ti, int tj, int kc) {
     Ctx& c = g_ctx;
     if (!c.initialised) return fail(E4C_ERR_STATE, "not initialised");
     if (!tile_available(ti, tj) || kc < 1) return fail(E4C_ERR_ARG, "tile shape not available");
+    c.tile_auto = false;
     c.tile_ti = ti;
     c.tile_tj = tj;
     c.tile_kc = kc;
@@ -1007,6 +1009,11 @@ int e4c_set_flux_runs(int i_faces, int jk_faces) {
 int e4c_get_tile(int* ti, int* tj, int* kc) {
     Ctx& c = g_ctx;
     if (!c.initialised) return fail(E4C_ERR_STATE, "not initialised");
+    if (c.tile_auto && !c.blocks.empty()) {
+        // the choice belongs to the current blocks
+        const int rc = c.prepare_fused();
+        if (rc != E4C_OK) return rc;
+    }
     if (ti) *ti = c.tile_ti;
     if (tj) *tj = c.tile_tj;
     if (kc) *kc = c.tile_kc;
@@ -1071,6 +1078,7 @@ int e4c_autotune(int nsteps, int* ti, int* tj, int* kc, double* ms_per_step) {
     std::vector<int> hs = c.all_blocks();
     const bool graphs = c.cfg.use_graphs != 0;
     c.cfg.use_graphs = 0;
+    c.tile_auto = false;
     for (auto& t : tiles) {
         for (int k : kcs) {
             c.tile_ti = t[0]; c.tile_tj = t[1]; c.tile_kc = k;

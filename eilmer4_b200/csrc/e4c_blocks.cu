@@ -2,6 +2,7 @@
 // per-step launch sequence.
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "e4c_internal.h"
@@ -225,6 +226,104 @@ int Ctx::build_block(int ni, int nj, int nk, const double* vtx, const int* bc,
     return E4C_OK;
 }
 
+int Ctx::fused_occupancy(int ti, int tj) const {
+    return cfg.precision == E4C_PREC_FP32_FLUX ? f32::fused_occupancy(cfg.flux_calculator, ti, tj)
+                                               : f64::fused_occupancy(cfg.flux_calculator, ti, tj);
+}
+
+// Tile shape and k-chunk of the fused stage for the current blocks: the pair
+// with the shortest modelled stage.  A work item costs its planes times the
+// tile's time per plane plus a start (its halo planes and the bottom faces);
+// the items go, costliest first, to the CTA slots of 148 SMs.  What the choice
+// trades: tall tiles and long chunks do the least extra work, but a block of
+// a few hundred thousand cells then leaves most SMs without an item, and a
+// ragged one ends in a nearly empty last round.
+//
+// plane: microseconds per full plane with the SM's CTAs all resident; alone:
+// the same for a CTA that has the SM to itself; start: microseconds per item.
+// Measured with HLLC on the 256^3 block (chunks of 32, 16, 8 and 4 planes) and
+// on four joined 48x36x40 blocks; only their ratios matter.  Against the fixed
+// 32x8 tile and 32-plane chunks (per stage, before -> chosen): the four
+// blocks 0.23 -> 0.11 ms, a 150x141x133 blast block 1.02 -> 0.93 ms, 64 uneven
+// blocks 2.04 -> 1.88 ms, 256^3 2.98 -> 2.80 ms.
+struct TileCost {
+    int ti, tj;
+    double plane, alone, start;
+};
+static const TileCost kTiles64[] = {{32, 14, 10.4, 10.4, 8.0}, {32, 8, 6.5, 6.5, 7.0},
+                                    {32, 4, 6.8, 4.5, 6.6},    {16, 16, 14.8, 9.5, 9.0},
+                                    {16, 8, 16.4, 6.5, 16.0}};
+static const TileCost kTiles32[] = {{32, 8, 5.3, 3.6, 7.5},  {32, 4, 4.7, 2.4, 10.0},
+                                    {32, 16, 5.7, 5.7, 9.0}, {16, 16, 13.2, 6.0, 4.6},
+                                    {16, 8, 14.8, 4.2, 6.0}};
+
+void Ctx::choose_tile() {
+    const bool f32_form = cfg.precision == E4C_PREC_FP32_FLUX;
+    const TileCost* tiles = f32_form ? kTiles32 : kTiles64;
+    const int ntiles = f32_form ? int(sizeof(kTiles32) / sizeof(TileCost))
+                                : int(sizeof(kTiles64) / sizeof(TileCost));
+    static const int chunks[] = {4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64};
+    int nsm = 148, max_nk = 0;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cfg.device);
+    for (const BlockHost& b : blocks)
+        if (b.fused) max_nk = std::max(max_nk, b.f.nk);
+    if (max_nk == 0) return;
+    double best = 1.0e300;
+    std::vector<double> cost, busy;
+    for (int q = 0; q < ntiles; ++q) {
+        const TileCost& t = tiles[q];
+        const int per_sm = fused_occupancy(t.ti, t.tj);
+        if (per_sm <= 0) continue;
+        for (int kc : chunks) {
+            cost.clear();
+            double total = 0.0, longest = 0.0;
+            long long items = 0;
+            for (const BlockHost& b : blocks)
+                if (b.fused)
+                    items += (long long)((b.f.ni + t.ti - 1) / t.ti) * ((b.f.nj + t.tj - 1) / t.tj) *
+                             ((b.f.nk + kc - 1) / kc);
+            // CTAs an SM holds at a time, and a plane's time then
+            const double share = per_sm > 1
+                ? std::min(1.0, std::max(0.0, double(items) / nsm - 1.0) / (per_sm - 1)) : 1.0;
+            const double plane = t.alone + (t.plane - t.alone) * share;
+            const long long slots = (long long)nsm * per_sm;
+            const bool exact = items <= 4096;
+            for (const BlockHost& b : blocks) {
+                if (!b.fused) continue;
+                const int tiles_i = (b.f.ni + t.ti - 1) / t.ti;
+                for (int j0 = 0; j0 < b.f.nj; j0 += t.tj)
+                    for (int k0 = 0; k0 < b.f.nk; k0 += kc) {
+                        // rows beyond the block are skipped; the plane's fixed
+                        // part (loads, edges, the barrier) stays
+                        const double rows = double(std::min(t.tj, b.f.nj - j0)) / t.tj;
+                        const double c = t.start + std::min(kc, b.f.nk - k0) * plane *
+                                                       (0.35 + 0.65 * rows);
+                        total += c * tiles_i;
+                        longest = std::max(longest, c);
+                        if (exact) cost.insert(cost.end(), size_t(tiles_i), c);
+                    }
+            }
+            double span = total / slots + longest;
+            if (exact) {
+                // costliest first, each to the slot that is free first
+                std::sort(cost.begin(), cost.end(), std::greater<double>());
+                busy.assign(size_t(std::min<long long>(slots, items)), 0.0);
+                for (double c : cost) {
+                    std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+                    busy.back() += c;
+                    std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+                }
+                span = *std::max_element(busy.begin(), busy.end());
+            }
+            if (span < best) {
+                best = span;
+                tile_ti = t.ti; tile_tj = t.tj; tile_kc = kc;
+            }
+            if (kc >= max_nk) break;
+        }
+    }
+}
+
 // (Re)build the device descriptor array of the fused blocks and the
 // persistent grid of the fused stage kernel.
 int Ctx::prepare_fused() {
@@ -239,6 +338,7 @@ int Ctx::prepare_fused() {
                                  stream));
         E4C_CUDA(cudaStreamSynchronize(stream));
     }
+    if (tile_auto) choose_tile();
     std::vector<FusedDesc> ds;
     long long items = 0;
     std::vector<int> desc_of(blocks.size(), -1);
@@ -316,9 +416,7 @@ int Ctx::prepare_fused() {
         E4C_CUDA(cudaStreamSynchronize(stream));
         int nsm = 148;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cfg.device);
-        const int per_sm = (cfg.precision == E4C_PREC_FP32_FLUX)
-                               ? f32::fused_occupancy(cfg.flux_calculator, tile_ti, tile_tj)
-                               : f64::fused_occupancy(cfg.flux_calculator, tile_ti, tile_tj);
+        const int per_sm = fused_occupancy(tile_ti, tile_tj);
         if (per_sm <= 0) return fail(E4C_ERR_UNSUPPORTED, "fused tile shape does not fit on the device");
         long long g = (long long)nsm * per_sm;
         fused_grid = int(std::min<long long>(g, items));

@@ -128,6 +128,7 @@ struct Ctx {
     long long fused_items = 0;
     bool descs_valid = false;
     int tile_ti = 32, tile_tj = 8, tile_kc = 32;
+    bool tile_auto = true;     // chosen by choose_tile, until e4c_set_tile or e4c_autotune
     int fused_grid = 0;
     int max_cells_fused = 0;
     // device list of block handles for the dt reduction
@@ -145,6 +146,8 @@ struct Ctx {
     void* dalloc(size_t bytes);
     void dfree(void* p);
     int prepare_fused();
+    void choose_tile();
+    int fused_occupancy(int ti, int tj) const;
     int set_hlist(const std::vector<int>& hs);
     bool uses_all_fused(const std::vector<int>& hs) const;
     void release();

@@ -392,7 +392,9 @@ int e4c_profile_steps(int nsteps, double* ms, int* launches);
 
 /* Tile shape of the fused stage kernel used for blocks with uniform
  * Cartesian geometry: ti x tj cells per CTA in the i-j plane, marching kc
- * planes in k.  Available (ti, tj): (32,8), (32,4), (16,8), (64,4), (16,16),
+ * planes in k; until it is called (or e4c_autotune), the shape and chunk are
+ * chosen for the blocks at hand by a model of the stage, again after e4c_init.
+ * Available (ti, tj): (32,8), (32,4), (16,8), (64,4), (16,16),
  * (32,16), (32,14). */
 int e4c_set_tile(int ti, int tj, int kc);
 int e4c_get_tile(int* ti, int* tj, int* kc);

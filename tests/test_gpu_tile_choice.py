@@ -1,0 +1,38 @@
+"""The fused stage's tile shape and k-chunk chosen for the blocks at hand
+(until e4c_set_tile or e4c_autotune fixes them): whatever is chosen gives the
+oracle's bits, a set shape stays, and a new context chooses again."""
+import pytest
+
+from eilmer4_b200 import workloads as W
+from tests.parity import FLUX, assert_same
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {(32, 14), (32, 8), (32, 4), (16, 16), (16, 8)}
+
+
+@pytest.mark.parametrize("sizes", [[(5, 4, 3)], [(40, 36, 30)], [(16, 100, 9)],
+                                   [(96, 17, 50), (12, 60, 16), (33, 29, 12)]])
+def test_chosen_tile(oracle, e4lib, sizes):
+    from eilmer4_b200.simcore import Simulation
+    blocks = [W.inflow_3d_block(*n, 3 + q, spacing=1.0 / 64.0) for q, n in enumerate(sizes)]
+    ref = oracle.OracleSim(oracle.default_config(dimensions=3, flux_calculator=FLUX["ausmdv"],
+                                                 n_threads=0))
+    with Simulation({"dimensions": 3, "flux_calculator": "ausmdv"}) as sim:
+        for b in blocks:
+            ref.set_flow(ref.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        ti, tj, kc = sim.get_tile()
+        assert (ti, tj) in SHAPES and kc >= 1
+        assert ref.run(8) == 0
+        sim.run(8)
+        assert sim.get_tile() == (ti, tj, kc)
+        for h in range(len(blocks)):
+            assert_same(sim.download(h)[1], ref.get_flow(h)[1], f"block {h}, tile {ti}x{tj}x{kc}")
+        sim.set_tile(64, 4, 7)
+        sim.run(1)
+        assert sim.get_tile() == (64, 4, 7)
+    with Simulation({"dimensions": 3, "flux_calculator": "ausmdv"}) as sim:
+        for b in blocks:
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        assert sim.get_tile() == (ti, tj, kc)
