@@ -27,7 +27,7 @@
 // (20 warps at 96 registers measured 6.7 ms/step where 16 took 5.8).
 // Measured on the 256^3 block, HLLC, per step: 7.53 ms for the per-face kernel
 // with the 32x8 tile and 32-plane chunks, 6.57 with its best tile (32x16);
-// 5.95 here with 32x8, 5.74 with 32x14.  128^3, 32x14 (ncu): 2,170
+// 5.98 here with 32x8, 5.59 with 32x14.  128^3, 32x14 (ncu): 2,170
 // instructions per warp and plane, 40 % of them FP64, 0.46 issued per cycle
 // and scheduler, stalls led by the FP64 chains (2.3 of 8.6 cycles) and the
 // barrier (1.6).
