@@ -122,7 +122,6 @@ static inline void launch_as(Ctx& c, int cls, int nkernels, F&& f) {
 // One stage over the given blocks (simcore.d:2325-2493 / 2529-2730).  All
 // fused blocks go through one launch of the fused stage kernel.
 void Ctx::enqueue_stage(const std::vector<int>& hs, int stage, int final_stage) {
-    launch_as(*this, E4C_KCLASS_OTHER, 1, [&] { launch_reset_bad(d_sim, stream); });
     bool any_fused = false;
     for (int h : hs) any_fused = any_fused || blocks[h].fused;
     if (any_fused)
@@ -162,8 +161,10 @@ void Ctx::enqueue_stage(const std::vector<int>& hs, int stage, int final_stage) 
         launch_as(*this, E4C_KCLASS_UPDATE, 1,
                   [&] { launch_update(b.v, d_sim, gas, stage, final_stage, stream); });
     }
+    // on the last stage of a step without chemistry it ends the step too
+    const int end_step = final_stage && !cfg.reacting;
     launch_as(*this, E4C_KCLASS_OTHER, 1,
-              [&] { launch_stage_check(d_sim, cfg.max_invalid_cells, stream); });
+              [&] { launch_stage_check(d_sim, cfg.max_invalid_cells, end_step, stream); });
 }
 
 void Ctx::enqueue_chemistry(const std::vector<int>& hs, const double* dt) {
@@ -205,8 +206,10 @@ void Ctx::enqueue_gasdynamic(const std::vector<int>& hs) {
     const int nstages = (cfg.gasdynamic_update_scheme == E4C_UPDATE_PC) ? 2 : 1;
     for (int s = 1; s <= nstages; ++s) enqueue_stage(hs, s, s == nstages);
     // chemistry_step(dt_global) after the gas-dynamic increment (simcore.d:903-907)
-    if (cfg.reacting) enqueue_chemistry(hs, &d_sim->dt_global);
-    launch_as(*this, E4C_KCLASS_OTHER, 1, [&] { launch_end_step(d_sim, stream); });
+    if (cfg.reacting) {
+        enqueue_chemistry(hs, &d_sim->dt_global);
+        launch_as(*this, E4C_KCLASS_OTHER, 1, [&] { launch_end_step(d_sim, stream); });
+    }
 }
 
 // dt control over the given blocks; accumulators are indexed by handle and
@@ -827,10 +830,10 @@ int e4c_stage(const int* h, int nb, int stage, double dt, int* bad_cells) {
                                  cudaMemcpyHostToDevice, c.stream));
     }
     c.enqueue_stage(hs, stage, stage == nstages);
-    if (stage == nstages) {
+    if (stage == nstages && c.cfg.reacting) {
         // chemistry_step(dt_global) after the gas-dynamic increment, then the
         // step's end (as e4c_gasdynamic_step)
-        if (c.cfg.reacting) c.enqueue_chemistry(hs, &c.d_sim->dt_global);
+        c.enqueue_chemistry(hs, &c.d_sim->dt_global);
         launch_end_step(c.d_sim, c.stream);
         c.launches += 1;
     }

@@ -171,6 +171,7 @@ __device__ __forceinline__ bool rhou_update(const FluxOpts& o, Prim<double, NSP>
 // (dir < 0: i faces, then j, then k, one index space).
 template <int NSP, int FLUX, int GAS>
 __global__ void k_flux(BlockView b, const SimDev* sim, FluxOpts o, int dir_arg) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     long long nd[3];
     for (int d = 0; d < 3; ++d)
@@ -458,6 +459,7 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
     static_assert(NSP == 1, "the row walk serves ideal-gas blocks");
     __shared__ double s_pf[2][kRowPrefetch][kRowThreads];
     const int tid = threadIdx.x;
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     // blocks whose frames are all signed unit axes: the round trips are exact
     // (up to the sign of a zero) and the reference copies instead of
@@ -651,6 +653,7 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
 // ---------------------------------------------------------------------------
 template <int NSP, int GAS>
 __global__ void k_update(BlockView b, SimDev* sim, GasConsts gas, int stage, int final_stage) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     constexpr int NSPC = NSP > 1 ? NSP : 0;
     constexpr int NV = 5 + NSPC;
@@ -786,7 +789,7 @@ __global__ void k_update(BlockView b, SimDev* sim, GasConsts gas, int stage, int
         if (T < 0.0 || T > 50000.0) ok = false;
         if (!ok) ++bad;
     }
-    if (bad) atomicAdd(&sim->bad_cells, bad);
+    if (bad) atomicAdd(&sim->bad_acc, bad);
 }
 
 // ---------------------------------------------------------------------------
@@ -872,6 +875,7 @@ template <int NSP, int NR>
 __global__ void k_chem_work(BlockView b, SimDev* sim, double T_frozen, const double* dt_p,
                             const int* work, const int* nwork, const double* guess,
                             unsigned long long* stats) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     const long long n = (long long)b.ni * b.nj * b.nk;
     const int nw = *nwork;

@@ -423,6 +423,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
     // one decision per CTA (another CTA may set the status while this one
     // starts): every thread leaves, or none
     __shared__ int s_stop;
+    pdl_wait();
     if (threadIdx.x == 0) s_stop = (sim->status != 0 || sim->finished) ? 1 : 0;
     __syncthreads();
     if (s_stop) return;
@@ -718,7 +719,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
         // from now on the sound speed comes from the decoded state
         for (int b = 0; b < nblocks; ++b) *descs[b].use_a0 = 0;
     }
-    if (bad) atomicAdd(&sim->bad_cells, bad);
+    if (bad) atomicAdd(&sim->bad_acc, bad);
 }
 
 // signal_frequency + block min/max of one fused block (fvcell.d:1624-1705,

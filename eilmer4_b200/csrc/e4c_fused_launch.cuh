@@ -31,9 +31,9 @@ static int launch_one(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, c
                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         attr_set = true;
     }
-    k_fused_stage<RT, FLUX, TI, TJ><<<L.grid, FusedThreads<TI, TJ>::total, smem, s>>>(
-        static_cast<const FusedDesc*>(L.descs), L.nblocks, L.nitems, L.kc, sim, gas, o, stage,
-        L.order);
+    launch_pdl(k_fused_stage<RT, FLUX, TI, TJ>, L.grid, FusedThreads<TI, TJ>::total, smem, s,
+               static_cast<const FusedDesc*>(L.descs), L.nblocks, L.nitems, L.kc, sim, gas, o,
+               stage, L.order);
     return 0;
 }
 
@@ -62,9 +62,9 @@ static int launch_ws(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, co
                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         attr_set = true;
     }
-    ws::k_fused_stage_ws<FLUX, TJ><<<L.grid, ws::Lay<TJ>::threads, smem, s>>>(
-        static_cast<const FusedDesc*>(L.descs), L.nblocks, L.nitems, L.kc, sim, gas, o, stage,
-        L.order);
+    launch_pdl(ws::k_fused_stage_ws<FLUX, TJ>, L.grid, ws::Lay<TJ>::threads, smem, s,
+               static_cast<const FusedDesc*>(L.descs), L.nblocks, L.nitems, L.kc, sim, gas, o,
+               stage, L.order);
     return 0;
 }
 
@@ -100,11 +100,11 @@ static int launch_ws64(const FusedLaunch& L, SimDev* sim, const GasConsts& gas, 
     if (FLUX == 3) {
         int gx = (L.max_cells + 255) / 256;
         if (gx > 148 * 16) gx = 148 * 16;
-        ws64::k_fused_shock<<<dim3(gx, L.nblocks), 256, 0, s>>>(descs, sim, gas,
-                                                                o.compression_tol, stage);
+        launch_pdl(ws64::k_fused_shock, dim3(gx, L.nblocks), 256, 0, s, descs, sim, gas,
+                   o.compression_tol, stage);
     }
-    ws64::k_fused_stage_ws64<FLUX, TJ><<<L.grid, ws64::Lay<TJ>::threads, smem, s>>>(
-        descs, L.nblocks, L.nitems, L.kc, sim, gas, o, stage, L.order);
+    launch_pdl(ws64::k_fused_stage_ws64<FLUX, TJ>, L.grid, ws64::Lay<TJ>::threads, smem, s, descs,
+               L.nblocks, L.nitems, L.kc, sim, gas, o, stage, L.order);
     return 0;
 }
 

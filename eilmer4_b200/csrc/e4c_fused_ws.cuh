@@ -401,6 +401,7 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
     // one decision per CTA (another CTA may set the status while this one
     // starts): every thread leaves, or none
     __shared__ int s_stop;
+    pdl_wait();
     if (threadIdx.x == 0) s_stop = (sim->status != 0 || sim->finished) ? 1 : 0;
     __syncthreads();
     if (s_stop) return;
@@ -731,7 +732,7 @@ k_fused_stage_ws(const FusedDesc* __restrict__ descs, int nblocks, long long nit
     if (stage == 2 && blockIdx.x == 0 && threadIdx.x == 0) {
         for (int b = 0; b < nblocks; ++b) *descs[b].use_a0 = 0;
     }
-    if (bad) atomicAdd(&sim->bad_cells, bad);
+    if (bad) atomicAdd(&sim->bad_acc, bad);
 }
 
 }  // namespace ws

@@ -266,6 +266,7 @@ k_fused_stage_ws64(const FusedDesc* __restrict__ descs, int nblocks, long long n
     // one decision per CTA (another CTA may set the status while this one
     // starts): every thread leaves, or none
     __shared__ int s_stop;
+    pdl_wait();
     if (threadIdx.x == 0) s_stop = (sim->status != 0 || sim->finished) ? 1 : 0;
     __syncthreads();
     if (s_stop) return;
@@ -628,7 +629,7 @@ k_fused_stage_ws64(const FusedDesc* __restrict__ descs, int nblocks, long long n
         // from now on the sound speed comes from the decoded state
         for (int b = 0; b < nblocks; ++b) *descs[b].use_a0 = 0;
     }
-    if (bad) atomicAdd(&sim->bad_cells, bad);
+    if (bad) atomicAdd(&sim->bad_acc, bad);
 }
 
 // Shock points of every fused block before a stage of the adaptive flux
@@ -641,6 +642,7 @@ k_fused_stage_ws64(const FusedDesc* __restrict__ descs, int nblocks, long long n
 // registers.  One block per blockIdx.y.
 __global__ void k_fused_shock(const FusedDesc* __restrict__ descs, const SimDev* sim,
                               GasConsts gas, double tol, int stage) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     const FusedDesc& d = descs[blockIdx.y];
     const double* W = static_cast<const double*>(stage == 1 ? d.WA : d.WB);

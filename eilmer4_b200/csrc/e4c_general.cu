@@ -304,6 +304,7 @@ __global__ void k_download(BlockView b, double* prim, double* cons) {
 // ---------------------------------------------------------------------------
 template <int NSP>
 __global__ void k_bc(BlockView b, const SimDev* sim) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     const int which = blockIdx.y;
     if (b.dim == 2 && which >= 4) return;
@@ -476,6 +477,7 @@ __device__ __forceinline__ int face_shock(const BlockView& b, const double* fg, 
 }
 
 __global__ void k_shock(BlockView b, const SimDev* sim, double tol) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     const long long n = (long long)b.ni * b.nj * b.nk;
     const size_t si = 1, sj = size_t(b.nidim), sk = size_t(b.nidim) * b.njdim;
@@ -634,21 +636,30 @@ __global__ void k_dt_finalize(SimDev* sim, const unsigned long long* acc, const 
     }
 }
 
-__global__ void k_stage_check(SimDev* sim, int max_invalid_cells) {
-    if (sim->status == 0 && sim->bad_cells > max_invalid_cells) {
-        sim->status = -4;
-        sim->status_step = sim->step;
-    }
-}
-
-__global__ void k_reset_bad(SimDev* sim) { sim->bad_cells = 0; }
-
-__global__ void k_end_step(SimDev* sim) {
+__device__ __forceinline__ void end_of_step(SimDev* sim) {
     if (sim->status != 0 || sim->finished) return;
     sim->time = sim->time + sim->dt_global;  // simcore.d:2951
     sim->step = sim->step + 1;
     if (sim->time >= sim->max_time) sim->finished = 1;  // simcore.d:1099
 }
+
+// The stage's invalid cells (simcore.d:2480-2493), its count taken over and
+// cleared for the next stage; on the last stage of a step without chemistry
+// the step's end as well.  (A launch of its own for each cost a small block
+// about a quarter of its step: 11 kernels a step -> 8.)
+__global__ void k_stage_check(SimDev* sim, int max_invalid_cells, int end_step) {
+    pdl_wait();
+    const int bad = sim->bad_acc;
+    sim->bad_acc = 0;
+    sim->bad_cells = bad;
+    if (sim->status == 0 && bad > max_invalid_cells) {
+        sim->status = -4;
+        sim->status_step = sim->step;
+    }
+    if (end_step) end_of_step(sim);
+}
+
+__global__ void k_end_step(SimDev* sim) { end_of_step(sim); }
 
 __global__ void k_begin_run(SimDev* sim, double max_time) {
     sim->max_time = max_time;
@@ -707,8 +718,8 @@ static int boundary_extent(const BlockView& b) {
 void launch_bc(const BlockView& b, const SimDev* sim, cudaStream_t s) {
     const int m = boundary_extent(b);
     dim3 grid((m + 127) / 128, b.dim == 3 ? 6 : 4);
-    if (b.nsp == 5) k_bc<5><<<grid, 128, 0, s>>>(b, sim);
-    else k_bc<1><<<grid, 128, 0, s>>>(b, sim);
+    if (b.nsp == 5) launch_pdl(k_bc<5>, grid, 128, 0, s, b, sim);
+    else launch_pdl(k_bc<1>, grid, 128, 0, s, b, sim);
 }
 
 void launch_bc_linear(const BlockView& b, SimDev* sim, const GasConsts& gas, cudaStream_t s) {
@@ -740,7 +751,7 @@ void launch_bc_flux(const BlockView& b, const SimDev* sim, const FluxOpts& o, cu
 
 void launch_shock(const BlockView& b, const SimDev* sim, double tol, cudaStream_t s) {
     long long n = (long long)b.ni * b.nj * b.nk;
-    k_shock<<<grid_for(n, 256), 256, 0, s>>>(b, sim, tol);
+    launch_pdl(k_shock, grid_for(n, 256), 256, 0, s, b, sim, tol);
 }
 
 // The velocity each interior cell of a block with general face frames holds
@@ -753,6 +764,7 @@ void launch_shock(const BlockView& b, const SimDev* sim, double tol, cudaStream_
 // its faces, so one thread per cell replays them once per stage for every
 // face that reads the cell.
 __global__ void k_replay_base(BlockView b, const SimDev* sim) {
+    pdl_wait();
     if (sim->status != 0 || sim->finished) return;
     const long long n = (long long)b.ni * b.nj * b.nk;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
@@ -781,7 +793,7 @@ __global__ void k_replay_base(BlockView b, const SimDev* sim) {
 void launch_replay_base(const BlockView& b, const SimDev* sim, cudaStream_t s) {
     const long long n = (long long)b.ni * b.nj * b.nk;
     const int T = 128;
-    k_replay_base<<<grid_for(n, T), T, 0, s>>>(b, sim);
+    launch_pdl(k_replay_base, grid_for(n, T), T, 0, s, b, sim);
 }
 
 // Faces per run of the row-walking flux kernel: i faces (runs of neighbouring
@@ -836,15 +848,15 @@ void launch_flux(const BlockView& b, const SimDev* sim, const FluxOpts& o, int d
         const int T = kRowThreads;
         const int g = grid_for(n, T);
         if (b.Vrt) {
-            if (o.flux == 1) k_flux_rows<1, 1, 0, true><<<g, T, 0, s>>>(b, sim, o, runs);
-            else if (o.flux == 2) k_flux_rows<1, 2, 0, true><<<g, T, 0, s>>>(b, sim, o, runs);
-            else if (o.flux == 3) k_flux_rows<1, 3, 0, true><<<g, T, 0, s>>>(b, sim, o, runs);
-            else k_flux_rows<1, 0, 0, true><<<g, T, 0, s>>>(b, sim, o, runs);
+            if (o.flux == 1) launch_pdl(k_flux_rows<1, 1, 0, true>, g, T, 0, s, b, sim, o, runs);
+            else if (o.flux == 2) launch_pdl(k_flux_rows<1, 2, 0, true>, g, T, 0, s, b, sim, o, runs);
+            else if (o.flux == 3) launch_pdl(k_flux_rows<1, 3, 0, true>, g, T, 0, s, b, sim, o, runs);
+            else launch_pdl(k_flux_rows<1, 0, 0, true>, g, T, 0, s, b, sim, o, runs);
         } else {
-            if (o.flux == 1) k_flux_rows<1, 1, 0, false><<<g, T, 0, s>>>(b, sim, o, runs);
-            else if (o.flux == 2) k_flux_rows<1, 2, 0, false><<<g, T, 0, s>>>(b, sim, o, runs);
-            else if (o.flux == 3) k_flux_rows<1, 3, 0, false><<<g, T, 0, s>>>(b, sim, o, runs);
-            else k_flux_rows<1, 0, 0, false><<<g, T, 0, s>>>(b, sim, o, runs);
+            if (o.flux == 1) launch_pdl(k_flux_rows<1, 1, 0, false>, g, T, 0, s, b, sim, o, runs);
+            else if (o.flux == 2) launch_pdl(k_flux_rows<1, 2, 0, false>, g, T, 0, s, b, sim, o, runs);
+            else if (o.flux == 3) launch_pdl(k_flux_rows<1, 3, 0, false>, g, T, 0, s, b, sim, o, runs);
+            else launch_pdl(k_flux_rows<1, 0, 0, false>, g, T, 0, s, b, sim, o, runs);
         }
         return;
     }
@@ -857,10 +869,10 @@ void launch_flux(const BlockView& b, const SimDev* sim, const FluxOpts& o, int d
     if (b.nsp == 5) {
         launch_flux_tp(b, sim, o, dir, g, T, s);
     } else {
-        if (o.flux == 1) k_flux<1, 1, 0><<<g, T, 0, s>>>(b, sim, o, dir);
-        else if (o.flux == 2) k_flux<1, 2, 0><<<g, T, 0, s>>>(b, sim, o, dir);
-        else if (o.flux == 3) k_flux<1, 3, 0><<<g, T, 0, s>>>(b, sim, o, dir);
-        else k_flux<1, 0, 0><<<g, T, 0, s>>>(b, sim, o, dir);
+        if (o.flux == 1) launch_pdl(k_flux<1, 1, 0>, g, T, 0, s, b, sim, o, dir);
+        else if (o.flux == 2) launch_pdl(k_flux<1, 2, 0>, g, T, 0, s, b, sim, o, dir);
+        else if (o.flux == 3) launch_pdl(k_flux<1, 3, 0>, g, T, 0, s, b, sim, o, dir);
+        else launch_pdl(k_flux<1, 0, 0>, g, T, 0, s, b, sim, o, dir);
     }
 }
 
@@ -869,7 +881,7 @@ void launch_update(const BlockView& b, SimDev* sim, const GasConsts& gas, int st
     long long n = (long long)b.ni * b.nj * b.nk;
     const int T = 128;
     if (b.nsp == 5) launch_update_tp(b, sim, gas, stage, final_stage, grid_for(n, T), T, s);
-    else k_update<1, 0><<<grid_for(n, T), T, 0, s>>>(b, sim, gas, stage, final_stage);
+    else launch_pdl(k_update<1, 0>, grid_for(n, T), T, 0, s, b, sim, gas, stage, final_stage);
 }
 
 // Per-cell chemistry step suggestion of the interior cells (i fastest) to or
@@ -943,9 +955,8 @@ void launch_check_uniform(const BlockView& b, int* flag, cudaStream_t s) {
     k_check_uniform<<<grid_for(n, 256), 256, 0, s>>>(b, flag);
 }
 
-void launch_reset_bad(SimDev* sim, cudaStream_t s) { k_reset_bad<<<1, 1, 0, s>>>(sim); }
-void launch_stage_check(SimDev* sim, int max_invalid, cudaStream_t s) {
-    k_stage_check<<<1, 1, 0, s>>>(sim, max_invalid);
+void launch_stage_check(SimDev* sim, int max_invalid, int end_step, cudaStream_t s) {
+    launch_pdl(k_stage_check, 1, 1, 0, s, sim, max_invalid, end_step);
 }
 void launch_end_step(SimDev* sim, cudaStream_t s) { k_end_step<<<1, 1, 0, s>>>(sim); }
 void launch_begin_run(SimDev* sim, double max_time, cudaStream_t s) {

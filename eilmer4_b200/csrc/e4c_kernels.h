@@ -20,6 +20,34 @@ struct FluxOpts {
     int row_run_i, row_run_jk;  // faces per run of k_flux_rows (0: chosen per block)
 };
 
+// Kernels of a time step are launched with programmatic stream serialization:
+// a kernel's CTAs may be placed while the last CTAs of the one before still
+// run, and wait (pdl_wait, their first statement) until it has completed and
+// its writes are visible.  Every such kernel waits before it reads or writes
+// device memory, so completion carries through the sequence.
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+// let the next kernel's CTAs be placed, then wait for the kernel before
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 // general-geometry FP64 path (e4c_general.cu)
 void launch_geometry(const BlockView& b, const double* vtx, cudaStream_t s);
 void launch_upload(const BlockView& b, const double* prim, cudaStream_t s);
@@ -52,8 +80,8 @@ void launch_dt(const BlockView& b, const SimDev* sim, double cfl_value, const do
 void launch_dt_finalize(SimDev* sim, const unsigned long long* acc, const int* hlist, int nb,
                         double cfl_allow, double dt_init, double dt_max, int check_cfl, int step0,
                         double* out_dt_allow, double* out_cfl_max, cudaStream_t s);
-void launch_reset_bad(SimDev* sim, cudaStream_t s);
-void launch_stage_check(SimDev* sim, int max_invalid, cudaStream_t s);
+// the end of a stage: its invalid cells checked, and (end_step) the step's end
+void launch_stage_check(SimDev* sim, int max_invalid, int end_step, cudaStream_t s);
 void launch_end_step(SimDev* sim, cudaStream_t s);
 void launch_begin_run(SimDev* sim, double max_time, cudaStream_t s);
 // compare every cell's and face's geometry with the first one; flag[0] != 0 if any

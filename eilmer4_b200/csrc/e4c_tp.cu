@@ -187,10 +187,10 @@ static int grid_for(long long n, int threads) {
 
 void launch_flux_tp(const BlockView& b, const SimDev* sim, const FluxOpts& o, int dir, int g,
                     int T, cudaStream_t s) {
-    if (o.flux == 1) k_flux<5, 1, 1><<<g, T, 0, s>>>(b, sim, o, dir);
-    else if (o.flux == 2) k_flux<5, 2, 1><<<g, T, 0, s>>>(b, sim, o, dir);
-    else if (o.flux == 3) k_flux<5, 3, 1><<<g, T, 0, s>>>(b, sim, o, dir);
-    else k_flux<5, 0, 1><<<g, T, 0, s>>>(b, sim, o, dir);
+    if (o.flux == 1) launch_pdl(k_flux<5, 1, 1>, g, T, 0, s, b, sim, o, dir);
+    else if (o.flux == 2) launch_pdl(k_flux<5, 2, 1>, g, T, 0, s, b, sim, o, dir);
+    else if (o.flux == 3) launch_pdl(k_flux<5, 3, 1>, g, T, 0, s, b, sim, o, dir);
+    else launch_pdl(k_flux<5, 0, 1>, g, T, 0, s, b, sim, o, dir);
 }
 
 static int boundary_cells(const BlockView& b) {
@@ -210,7 +210,7 @@ void launch_ghost_defaults_tp(const BlockView& b, const GasConsts& gas, cudaStre
 
 void launch_update_tp(const BlockView& b, SimDev* sim, const GasConsts& gas, int stage,
                       int final_stage, int g, int T, cudaStream_t s) {
-    k_update<5, 1><<<g, T, 0, s>>>(b, sim, gas, stage, final_stage);
+    launch_pdl(k_update<5, 1>, g, T, 0, s, b, sim, gas, stage, final_stage);
 }
 
 void launch_seed_active_list(const BlockView& b, double T_frozen, double dt, int* list, int* count,
@@ -242,7 +242,7 @@ int launch_chem_work(const BlockView& b, SimDev* sim, double T_frozen, const dou
     // 64-thread CTAs per SM strides over it
     long long g = (n + 63) / 64;
     if (g > 148 * 16) g = 148 * 16;
-    k_chem_work<5, 5><<<int(g), 64, 0, s>>>(b, sim, T_frozen, dt, work, nwork, guess, stats);
+    launch_pdl(k_chem_work<5, 5>, int(g), 64, 0, s, b, sim, T_frozen, dt, work, nwork, guess, stats);
     return 0;
 }
 

@@ -134,9 +134,9 @@ struct SimDev {
     int step;
     int status;                     // first error code seen, 0 if none
     int status_step;                // step at which it was seen
-    int bad_cells;                  // invalid cells counted in the last stage
+    int bad_cells;                  // invalid cells of the last stage (k_stage_check)
     int finished;                   // set when time >= max_time
-    int pad_;
+    int bad_acc;                    // invalid cells of the stage in progress
     unsigned int item_next[2];      // work-item counters of the fused stages 1 and 2
     unsigned int pad2_[2];
 };
