@@ -298,9 +298,29 @@ k_fused_stage_ws64(const FusedDesc* __restrict__ descs, int nblocks, long long n
     const bool a_ok = gR >= 0.0 && isfinite(gR * 50000.0);
     int bad = 0;
     auto slot_of = [&](int kk) { return ring + ((kk + 8) & 3) * (5 * NPOS); };
-    // positions the boundary conditions never fill (beyond the second ghost
-    // layer of a partial tile) are read by lanes whose results are not used
-    for (int e = threadIdx.x; e < L::words; e += blockDim.x) sm64[e] = 0.0;
+    // Positions the boundary conditions never fill (the block's corners, beyond
+    // the second ghost layer of a partial tile) are read by lanes whose results
+    // are not used.  They start as a cell of the first block: with zeros there
+    // the density, pressure and sound speed of such a lane are out of the
+    // batched quotients' range, and its whole warp goes through the plain
+    // divisions as well (flux_ieee), every plane.  AUSMDV, 125x122x151 (29 of
+    // 32 lanes in the last tile): 2.96 ms/step with zeros, 1.13 with a cell (the
+    // per-face kernel's 32x8 tile: 1.74); over 24 layouts of partial tiles the
+    // step is 0.57 of that with zeros (Hanel 0.75, adaptive 0.69, HLLC, whose
+    // supersonic faces need no quotient, 1.00).  A gas at rest in its place made
+    // HLLC take its subsonic side for those lanes (1.03).
+    double first[5];
+    {
+        const double* c = static_cast<const double*>(stage == 1 ? descs[0].WA : descs[0].WB);
+        const size_t n = size_t(descs[0].ni) * descs[0].nj * descs[0].nk;
+#pragma unroll
+        for (int f = 0; f < 5; ++f) first[f] = c[f * n];
+    }
+    for (int e = threadIdx.x; e < L::words - L::o_hj; e += blockDim.x) Hj[e] = 0.0;
+    for (int e = threadIdx.x; e < NPOS; e += blockDim.x) {
+#pragma unroll
+        for (int q = 0; q < 20; ++q) ring[q * NPOS + e] = first[q % 5];
+    }
 
     for (;;) {
         __syncthreads();

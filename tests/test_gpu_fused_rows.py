@@ -82,3 +82,32 @@ def test_options(oracle, e4lib, kw):
 def test_joined_blocks(oracle, e4lib, parts, flux):
     blocks, conns = W.split_block(blast(40, 30, 12), 3, parts)
     both(oracle, blocks, conns, flux, 10, (32, 14, 8))
+
+
+def test_partial_tiles_cost_no_more_than_full_ones(e4lib):
+    """125 cells in i fill the same four tiles as 128: the three idle lanes of
+    the last tile must not slow its warps down (left with an unphysical state
+    they took every face's plain divisions: 2.6 times the step)."""
+    import torch
+
+    from eilmer4_b200.simcore import Simulation
+
+    def ms_per_step(ni):
+        b = W.inflow_3d_block(ni, 112, 64, 5, spacing=1.0 / 64.0)
+        with Simulation({"dimensions": 3, "flux_calculator": "ausmdv"}) as sim:
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+            sim.set_tile(32, 14, 16)
+            sim.run(5)
+            s = torch.cuda.ExternalStream(sim.stream_handle())
+            best = 1.0e9
+            for _ in range(3):
+                e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                e[0].record(s)
+                sim.run(20)
+                e[1].record(s)
+                torch.cuda.synchronize()
+                best = min(best, e[0].elapsed_time(e[1]) / 20)
+            return best
+
+    full, partial = ms_per_step(128), ms_per_step(125)
+    assert partial < 1.4 * full, (partial, full)
