@@ -119,8 +119,22 @@ __device__ __forceinline__ void load_frame(const double* fg, size_t npad, size_t
     fr.t2 = {fg[6 * npad + f], fg[7 * npad + f], fg[8 * npad + f]};
 }
 
-// rho, velocity and u of a face's two states from its four stencil cells
-template <int NSP>
+// Scalars whose limiter quotients share a batch: a batch keeps its operands
+// live, so its width is what the kernel's registers hold without costing
+// resident warps.  k_flux: 3 (126 registers, 4 CTAs of 128 threads per SM; all
+// 5 at once took 164 and 3 CTAs: a 2048x1024 block 985 against 866 us/step with
+// AUSMDV, 946 against 830 with HLLC, 928 and 877 with one division after
+// another; the 5-species form spills 988 against 1,212 B, its time the same).
+// k_flux_rows: 1 (at most 168 registers, 3 CTAs of 128 threads per SM; 5 took
+// 230-240, 2 and 3 take up to 174 and 216, all 2 CTAs in some of its forms):
+// us/step with 5 -> 1 and with one division after another, curvilinear
+// 40x36x30 HLLC 117 -> 106 (106), 128^3 AUSMDV 1,653 -> 1,560 (1,658) and
+// adaptive 1,955 -> 1,808 (1,897), stretched 118x90x70 AUSMDV 468 -> 449 (500).
+constexpr int kFluxBatch = 3, kRowBatch = 1;
+
+// rho, velocity and u of a face's two states from its four stencil cells (B:
+// scalars per batch of quotients)
+template <int NSP, int B>
 __device__ __forceinline__ void interp_face(const L2R2<double>& r, bool lim, bool clip,
                                             const Prim<double, NSP>& a, const Prim<double, NSP>& b,
                                             const Prim<double, NSP>& c, const Prim<double, NSP>& d,
@@ -130,12 +144,12 @@ __device__ __forceinline__ void interp_face(const L2R2<double>& r, bool lim, boo
                             {c.vel.x, c.vel.y, c.vel.z, c.rho, c.u},
                             {d.vel.x, d.vel.y, d.vel.z, d.rho, d.u}};
     double L[5], R[5];
-    r.interp<5>(lim, clip, q, L, R);
+    r.interp<5, B>(lim, clip, q, L, R);
     Lf.vel = {L[0], L[1], L[2]}; Lf.rho = L[3]; Lf.u = L[4];
     Rt.vel = {R[0], R[1], R[2]}; Rt.rho = R[3]; Rt.u = R[4];
 }
 // and the mass fractions
-template <int NSP>
+template <int NSP, int B>
 __device__ __forceinline__ void interp_massf(const L2R2<double>& r, bool lim, bool clip,
                                              const Prim<double, NSP>& a, const Prim<double, NSP>& b,
                                              const Prim<double, NSP>& c, const Prim<double, NSP>& d,
@@ -145,7 +159,7 @@ __device__ __forceinline__ void interp_massf(const L2R2<double>& r, bool lim, bo
     for (int s = 0; s < NSP; ++s) {
         q[0][s] = a.massf[s]; q[1][s] = b.massf[s]; q[2][s] = c.massf[s]; q[3][s] = d.massf[s];
     }
-    r.interp<NSP>(lim, clip, q, Lf.massf, Rt.massf);
+    r.interp<NSP, B>(lim, clip, q, Lf.massf, Rt.massf);
 }
 
 // update_thermo_from_rhou of a reconstructed state: ideal gas, or the
@@ -224,9 +238,9 @@ __global__ void k_flux(BlockView b, const SimDev* sim, FluxOpts o, int dir_arg) 
                 const double* len = b.cgeom + size_t(1 + dir) * b.npad;
                 L2R2<double> r;
                 r.prepare(len[cL1], len[cL0], len[cR0], len[cR1]);
-                interp_face<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                interp_face<NSP, kFluxBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                 if (NSP > 1) {
-                    interp_massf<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                    interp_massf<NSP, kFluxBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                     if (!scale_mass_fractions<double, NSP>(Lf.massf))
                         for (int q = 0; q < NSP; ++q) Lf.massf[q] = sL0.massf[q];
                     if (!scale_mass_fractions<double, NSP>(Rt.massf))
@@ -588,9 +602,9 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
             {
                 L2R2<double> r;
                 r.prepare(wl[0], wl[1], wl[2], wl[3]);
-                interp_face<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                interp_face<NSP, kRowBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                 if (NSP > 1) {
-                    interp_massf<NSP>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                    interp_massf<NSP, kRowBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                     if (!scale_mass_fractions<double, NSP>(Lf.massf))
                         for (int q = 0; q < NSP; ++q) Lf.massf[q] = sL0.massf[q];
                     if (!scale_mass_fractions<double, NSP>(Rt.massf))

@@ -246,42 +246,49 @@ struct L2R2 {
         two_R0_R1 = (R(2.0) * lenR0_ + lenR1);
     }
     // interp_l2r2_scalar, onedinterp.d:136-162 (van Albada, epsilon 1e-12 at
-    // :22), for N scalars at once: q[0..3] the values in the cells L1, L0, R0,
-    // R1.  The 2 N limiter quotients are one batch (fdiv_va).
-    template <int N>
+    // :22), for N scalars: q[0..3] the values in the cells L1, L0, R0, R1.
+    // The limiter quotients go in batches of 2 B (fdiv_va).
+    template <int N, int B = N>
     __device__ __forceinline__ void interp(bool limiter, bool clip, const R (&q)[4][N], R (&qL)[N],
                                            R (&qR)[N]) const {
+        interp_from<N, B, 0>(limiter, clip, q, qL, qR);
+    }
+    template <int N, int B, int I0>
+    __device__ __forceinline__ void interp_from(bool limiter, bool clip, const R (&q)[4][N],
+                                                R (&qL)[N], R (&qR)[N]) const {
+        constexpr int M = N - I0 < B ? N - I0 : B;
         const R eps = R(1.0e-12);
-        R dm[N], d0[N], dp[N], s[2 * N];
+        R dm[M], d0[M], dp[M], s[2 * M];
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            dm[i] = (q[1][i] - q[0][i]) * tw_L0L1;
-            d0[i] = (q[2][i] - q[1][i]) * tw_R0L0;
-            dp[i] = (q[3][i] - q[2][i]) * tw_R1R0;
-            s[i] = s[N + i] = R(1.0);
+        for (int i = 0; i < M; ++i) {
+            dm[i] = (q[1][I0 + i] - q[0][I0 + i]) * tw_L0L1;
+            d0[i] = (q[2][I0 + i] - q[1][I0 + i]) * tw_R0L0;
+            dp[i] = (q[3][I0 + i] - q[2][I0 + i]) * tw_R1R0;
+            s[i] = s[M + i] = R(1.0);
         }
         if (limiter) {
-            R nu[2 * N], de[2 * N];
+            R nu[2 * M], de[2 * M];
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
+            for (int i = 0; i < M; ++i) {
                 nu[i] = dm[i] * d0[i] + fabs(dm[i] * d0[i]) + eps;
                 de[i] = dm[i] * dm[i] + d0[i] * d0[i] + eps;
-                nu[N + i] = d0[i] * dp[i] + fabs(d0[i] * dp[i]) + eps;
-                de[N + i] = d0[i] * d0[i] + dp[i] * dp[i] + eps;
+                nu[M + i] = d0[i] * dp[i] + fabs(d0[i] * dp[i]) + eps;
+                de[M + i] = d0[i] * d0[i] + dp[i] * dp[i] + eps;
             }
-            fdiv_va<2 * N>(nu, de, s);
+            fdiv_va<2 * M>(nu, de, s);
         }
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            R l = q[1][i] + s[i] * aL0 * (d0[i] * two_L0_L1 + dm[i] * lenR0);
-            R r = q[2][i] - s[N + i] * aR0 * (dp[i] * lenL0 + d0[i] * two_R0_R1);
+        for (int i = 0; i < M; ++i) {
+            R l = q[1][I0 + i] + s[i] * aL0 * (d0[i] * two_L0_L1 + dm[i] * lenR0);
+            R r = q[2][I0 + i] - s[M + i] * aR0 * (dp[i] * lenL0 + d0[i] * two_R0_R1);
             if (clip) {
-                l = clip_to_limits(l, q[1][i], q[2][i]);
-                r = clip_to_limits(r, q[1][i], q[2][i]);
+                l = clip_to_limits(l, q[1][I0 + i], q[2][I0 + i]);
+                r = clip_to_limits(r, q[1][I0 + i], q[2][I0 + i]);
             }
-            qL[i] = l;
-            qR[i] = r;
+            qL[I0 + i] = l;
+            qR[I0 + i] = r;
         }
+        if constexpr (I0 + M < N) interp_from<N, B, I0 + M>(limiter, clip, q, qL, qR);
     }
     // With uniform cell lengths (tw_L0L1 == tw_R0L0 == tw_R1R0) the sL of a
     // face and the sR of the face before it are one van Albada value of their
