@@ -185,6 +185,19 @@ __device__ __forceinline__ void cell_pressure(Prim<R, 1>& s, const GasConsts& ga
     s.p = s.rho * R(gas.Rgas) * T;
 }
 
+// The FP32-flux form keeps its cheap FP32 divisions scalar by scalar, and the
+// update's FP64 reciprocals in the compiler's division: all five scalars at once
+// and an out-of-line fallback cost it 2-4 % at its 64 registers (160x128x160,
+// 16x8 tile, AUSMDV 890 against 846 us/step; HLLC 818 and 789; 16x16 843 and
+// 819).  In FP64 the batch is the faster one (128^3, 16x16, HLLC 1,028 -> 985).
+template <typename R>
+constexpr int kFaceBatch = sizeof(R) == 8 ? 5 : 1;
+template <typename R>
+__device__ __forceinline__ double reciprocal(double x) {
+    if constexpr (sizeof(R) == 8) return fdiv(1.0, x);
+    else return 1.0 / x;
+}
+
 // Reconstruction + flux of one face from four cells (general-path semantics,
 // sfluidblock.d:2190-2344 with onedinterp.d:435-585 and fluxcalc.d:26-128),
 // with the face frame of direction DIR applied as a permutation.
@@ -224,7 +237,7 @@ __device__ __forceinline__ void face_flux(Prim<R, 1> sL1, Prim<R, 1> sL0, Prim<R
                                {sR0.vel.x, sR0.vel.y, sR0.vel.z, sR0.rho, sR0.u},
                                {sR1.vel.x, sR1.vel.y, sR1.vel.z, sR1.rho, sR1.u}};
             R l[5], r[5];
-            w.template interp<5>(lim, clip, q, l, r);
+            w.template interp<5, kFaceBatch<R>>(lim, clip, q, l, r);
             Lf.vel = {l[0], l[1], l[2]}; Lf.rho = l[3]; Lf.u = l[4];
             Rt.vel = {r[0], r[1], r[2]}; Rt.rho = r[3]; Rt.u = r[4];
         }
@@ -651,7 +664,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
                     s -= double(Fbot[v]) * (-1.0 * aT);
                     integral[v] = s;
                 }
-                const double vol_inv = fdiv(1.0, d.vol);
+                const double vol_inv = reciprocal<R>(d.vol);
                 const size_t c = (size_t(k) * d.nj + j) * d.ni + i;
                 double Un[5];
                 if (stage == 1) {
@@ -675,7 +688,7 @@ k_fused_stage(const FusedDesc* __restrict__ descs, int nblocks, long long nitems
                     if (atomicCAS(&sim->status, 0, -5) == 0) sim->status_step = sim->step;
                     ok = false;
                 } else {
-                    const double dinv = fdiv(1.0, rho);
+                    const double dinv = reciprocal<R>(rho);
                     vx = Un[1] * dinv; vy = Un[2] * dinv; vz = Un[3] * dinv;
                     u = Un[4] * dinv;
                     const double ke = 0.5 * (vx * vx + vy * vy + vz * vz);
