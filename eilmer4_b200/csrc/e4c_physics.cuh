@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "e4c_quotients.cuh"
 #include "e4c_types.h"
 
 namespace e4c {
@@ -58,146 +59,6 @@ struct Prim {
     V3<R> vel;
     R massf[NSP];
 };
-
-// ---------------------------------------------------------------------------
-// Correctly rounded FP64 quotients without a branch per division.
-//
-// The compiler's a / b carries its own range test and slow-path call, so
-// independent divisions run one after the other, each a chain of dependent
-// FP64 operations: the reconstruction's limiter values alone are five to
-// twenty such chains.  Here one integer test covers a whole batch; inside the
-// tested range every quotient is
-//   y0 = rcp.approx (about 2^-20), two Newton steps -> y = 1/b rounded from a
-//   value within 2^-80 of it,
-//   q = a y, then twice: r = a - q b, q = q + r y,
-// and the last step is RN(a/b) by the argument of Markstein's theorem (P. W.
-// Markstein, IBM J. Res. Develop. 34(1), 1990): q is then within half an ulp
-// (and 2^-50 of it) of a/b and r exact, so the sum before rounding misses a/b
-// by at most ulp(q)/2 2^-53 (m/2)(1 + 2^-26), m the mantissa of b, while a/b
-// is at least ulp(q)/2 2^-53 (2/m) away from any midpoint of two doubles:
-// the result is the division's for m^2 < 4 (1 - 2^-26).  Divisors with the top
-// 20 mantissa bits set are left to the compiler's division (div_ieee), as are
-// operands outside the range (zero or huge divisors, infinities, NaN).
-// tests/test_quotients.py restates the steps in C and checks them against
-// IEEE division, the hardest dividends of each divisor among them.
-// ---------------------------------------------------------------------------
-static __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
-
-__device__ __forceinline__ unsigned abs_hi(double x) {
-    return unsigned(__double2hiint(x)) & 0x7fffffffu;
-}
-// 2^-200 <= |x| < 2^200 (the high words of the two ends)
-__device__ __forceinline__ bool quot_range(double x) {
-    return abs_hi(x) - 0x33700000u < 0x19000000u;
-}
-// the same, or zero (a dividend)
-__device__ __forceinline__ bool quot_range0(double x) { return quot_range(x) || x == 0.0; }
-// a divisor whose top 20 mantissa bits are all set
-__device__ __forceinline__ bool top_mantissa(double x) {
-    return (unsigned(__double2hiint(x)) & 0xfffffu) == 0xfffffu;
-}
-__device__ __forceinline__ bool quot_divisor(double x) { return quot_range(x) && !top_mantissa(x); }
-
-// 1/b for quot, b a quot_divisor
-__device__ __forceinline__ double rcp_q(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = fma(-b, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-b, y, 1.0);
-    return fma(y, e, y);
-}
-// 1/b for quot, b in quot_range with any mantissa
-__device__ __forceinline__ double rcp_any(double b) {
-    return top_mantissa(b) ? div_ieee(1.0, b) : rcp_q(b);
-}
-// a / b from y = rcp_q(b), or y = RN(1/b)
-__device__ __forceinline__ double quot(double a, double b, double y) {
-    double q = a * y;
-    double r = fma(-q, b, a);
-    q = fma(r, y, q);
-    r = fma(-q, b, a);
-    return fma(r, y, q);
-}
-// one quotient, any operands
-__device__ __forceinline__ double fdiv(double a, double b) {
-    if (quot_divisor(b) && quot_range0(a)) return quot(a, b, rcp_q(b));
-    return div_ieee(a, b);
-}
-__device__ __forceinline__ float fdiv(float a, float b) { return a / b; }
-// N independent quotients, any operands
-template <int N>
-__device__ __forceinline__ void fdivs(const double* a, const double* b, double* q) {
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < N; ++i) ok = ok && quot_divisor(b[i]) && quot_range0(a[i]);
-    if (ok) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) q[i] = quot(a[i], b[i], rcp_q(b[i]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) q[i] = div_ieee(a[i], b[i]);
-    }
-}
-template <int N>
-__device__ __forceinline__ void fdivs(const float* a, const float* b, float* q) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) q[i] = a[i] / b[i];
-}
-// N quotients n / d of van Albada values: 1e-12 <= n <= d (1 + 2^-52) wherever
-// d is finite, so the divisors' upper end is the only test of range
-template <int N>
-__device__ __forceinline__ void fdiv_va(const double* n, const double* d, double* q) {
-    unsigned top = 0u, man = 0u;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const unsigned h = unsigned(__double2hiint(d[i]));
-        top = max(top, h);
-        man = max(man, h & 0xfffffu);
-    }
-    // every d below 2^200 (and not negative, infinite or NaN)
-    if (top < 0x4c700000u && man < 0xfffffu) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) q[i] = quot(n[i], d[i], rcp_q(d[i]));
-    } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) q[i] = div_ieee(n[i], d[i]);
-    }
-}
-template <int N>
-__device__ __forceinline__ void fdiv_va(const float* n, const float* d, float* q) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) q[i] = n[i] / d[i];
-}
-// a / b with y from the caller's batch (FAST: y = rcp_or(b)), or the plain division
-template <bool FAST>
-__device__ __forceinline__ double quot_or(double a, double b, double y) {
-    if constexpr (FAST) return quot(a, b, y);
-    else return a / b;
-}
-template <bool FAST>
-__device__ __forceinline__ float quot_or(float a, float b, float) {
-    return a / b;
-}
-template <bool FAST>
-__device__ __forceinline__ double rcp_or(double b) {
-    if constexpr (FAST) return rcp_q(b);
-    else return 0.0;
-}
-template <bool FAST>
-__device__ __forceinline__ float rcp_or(float) {
-    return 0.0f;
-}
-// (a divisor formed inside the batch: its mantissa is tested here)
-template <bool FAST>
-__device__ __forceinline__ double rcp_or_any(double b) {
-    if constexpr (FAST) return rcp_any(b);
-    else return 0.0;
-}
-template <bool FAST>
-__device__ __forceinline__ float rcp_or_any(float) {
-    return 0.0f;
-}
 
 // RN(d / a) < tol for a shock detector's compression test, the quotient
 // formed only where the outcome is not already certain: with a > 0 and
@@ -511,13 +372,16 @@ __device__ __forceinline__ void ausmdv_with(const Prim<R, NSP>& Lf, const Prim<R
 }
 
 // Whether a face's states keep every operand of the AUSMDV and Hanel fluxes'
-// quotients in the batched form's range.
+// quotients in the batched form's range.  A normal velocity of -0 (beside a wall,
+// or in a gas at rest) may come out of u / a as +0: both fluxes only add that
+// quotient to 1 or 2, and compare its magnitude.  Their other dividends are not
+// -0, but for -(uR - am)^2 at uR = am, to whose multiple a +0 is added.
 template <int NSP>
 __device__ __forceinline__ bool flux_range(const Prim<double, NSP>& Lf, const Prim<double, NSP>& Rt) {
     return quot_divisor(Lf.rho) && quot_divisor(Rt.rho) && quot_divisor(Lf.p) &&
            quot_divisor(Rt.p) && quot_divisor(Lf.a) && quot_divisor(Rt.a) &&
-           quot_range0(Lf.vel.x) && !top_mantissa(Lf.vel.x) && quot_range0(Rt.vel.x) &&
-           !top_mantissa(Rt.vel.x);
+           (quot_range(Lf.vel.x) || Lf.vel.x == 0.0) && !top_mantissa(Lf.vel.x) &&
+           (quot_range(Rt.vel.x) || Rt.vel.x == 0.0) && !top_mantissa(Rt.vel.x);
 }
 
 // The two fluxes with plain divisions, for states outside that range (out of
