@@ -253,9 +253,15 @@ struct TileCost {
 static const TileCost kTiles64[] = {{32, 14, 10.4, 10.4, 8.0}, {32, 8, 6.5, 6.5, 7.0},
                                     {32, 4, 6.8, 4.5, 6.6},    {16, 16, 14.8, 9.5, 9.0},
                                     {16, 8, 16.4, 6.5, 16.0}};
-static const TileCost kTiles32[] = {{32, 8, 5.3, 3.6, 7.5},  {32, 4, 4.7, 2.4, 10.0},
-                                    {32, 16, 5.7, 5.7, 9.0}, {16, 16, 13.2, 6.0, 4.6},
-                                    {16, 8, 14.8, 4.2, 6.0}};
+// The FP32-flux form chooses among the edge-warp kernel's shapes only.  The
+// per-face kernel that serves 16- and 64-wide tiles rounds differently (scaled
+// differences, FP64 sums of the face fluxes): with its shapes among the choices
+// a block's results depended on which kernel the other blocks' sizes selected.
+static const TileCost kTiles32[] = {{32, 8, 5.3, 3.6, 7.5}, {32, 4, 4.7, 2.4, 10.0},
+                                    {32, 16, 5.7, 5.7, 9.0}};
+// Not among the choices, slower wherever they were measured: FP64 32x16 and
+// 64x4 (the per-face kernel; 128^3 AUSMDV 1.12 and 1.83 ms/step against 1.07
+// with 32x8), FP32-flux 32x14 (256^3 HLLC 2.95 against 2.48 with 32x8).
 
 void Ctx::choose_tile() {
     const bool f32_form = cfg.precision == E4C_PREC_FP32_FLUX;

@@ -395,7 +395,12 @@ int e4c_profile_steps(int nsteps, double* ms, int* launches);
  * planes in k; until it is called (or e4c_autotune), the shape and chunk are
  * chosen for the blocks at hand by a model of the stage, again after e4c_init.
  * Available (ti, tj): (32,8), (32,4), (16,8), (64,4), (16,16),
- * (32,16), (32,14). */
+ * (32,16), (32,14).  FP64 results do not depend on shape or chunk, bit for bit.
+ * Those of the FP32-flux form do, within FP32 rounding: on the chunk length (a
+ * face between two chunks), and on whether the shape is 32 cells wide (another
+ * kernel).  The automatic choice takes 32-wide shapes only, but its chunk
+ * follows the blocks, so adding a block can change another's last FP32 digits;
+ * e4c_set_tile fixes both. */
 int e4c_set_tile(int ti, int tj, int kc);
 int e4c_get_tile(int* ti, int* tj, int* kc);
 

@@ -36,3 +36,16 @@ def test_chosen_tile(oracle, e4lib, sizes):
         for b in blocks:
             sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
         assert sim.get_tile() == (ti, tj, kc)
+
+
+@pytest.mark.parametrize("sizes", [[(48, 96, 96), (48, 96, 96)], [(96, 96, 96)], [(112, 112, 114)],
+                                   [(40, 88, 91)], [(16, 64, 48)] * 9])
+def test_fp32_choice_keeps_the_edge_warp_kernel(e4lib, sizes):
+    """16-wide tiles are another kernel with other rounding: whatever the layout,
+    the FP32-flux form's own choice is 32 wide."""
+    from eilmer4_b200.simcore import Simulation
+    with Simulation({"dimensions": 3, "flux_calculator": "hllc"}, precision="fp32_flux") as sim:
+        for n in sizes:
+            b = W.inflow_3d_block(*n, 3, spacing=1.0 / 64.0)
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        assert sim.get_tile()[0] == 32
