@@ -332,6 +332,7 @@ int e4c_init(const e4c_config* cfg) {
     c.fopts.row_run_i = 0;
     c.fopts.row_run_jk = 0;
     c.tile_auto = true;
+    c.tile_ti = 32; c.tile_tj = 8; c.tile_kc = 32;
     E4C_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     E4C_CUDA(cudaStreamCreateWithFlags(&c.h2d_stream, cudaStreamNonBlocking));
     E4C_CUDA(cudaStreamCreateWithFlags(&c.d2h_stream, cudaStreamNonBlocking));
@@ -1012,11 +1013,9 @@ int e4c_set_flux_runs(int i_faces, int jk_faces) {
 int e4c_get_tile(int* ti, int* tj, int* kc) {
     Ctx& c = g_ctx;
     if (!c.initialised) return fail(E4C_ERR_STATE, "not initialised");
-    if (c.tile_auto && !c.blocks.empty()) {
-        // the choice belongs to the current blocks
-        const int rc = c.prepare_fused();
-        if (rc != E4C_OK) return rc;
-    }
+    // the choice belongs to the current blocks (host arithmetic only: nothing is
+    // allocated, queued or waited for)
+    if (c.tile_auto && !c.descs_valid) c.choose_tile();
     if (ti) *ti = c.tile_ti;
     if (tj) *tj = c.tile_tj;
     if (kc) *kc = c.tile_kc;

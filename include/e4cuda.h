@@ -402,6 +402,8 @@ int e4c_profile_steps(int nsteps, double* ms, int* launches);
  * follows the blocks, so adding a block can change another's last FP32 digits;
  * e4c_set_tile fixes both. */
 int e4c_set_tile(int ti, int tj, int kc);
+/* The shape and chunk set, or those the model chooses for the blocks created
+ * so far ((32,8) and 32 without any).  Queues nothing and does not wait. */
 int e4c_get_tile(int* ti, int* tj, int* kc);
 
 /* Faces per thread of the row-walking flux kernel that 3-D ideal-gas blocks

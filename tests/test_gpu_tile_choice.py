@@ -49,3 +49,26 @@ def test_fp32_choice_keeps_the_edge_warp_kernel(e4lib, sizes):
             b = W.inflow_3d_block(*n, 3, spacing=1.0 / 64.0)
             sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
         assert sim.get_tile()[0] == 32
+
+
+def test_get_tile_does_not_wait(e4lib):
+    """Asking for the automatic choice while the library's stream is busy."""
+    import time
+
+    import torch
+
+    from eilmer4_b200.simcore import Simulation
+    with Simulation({"dimensions": 3, "flux_calculator": "hllc"}) as sim:
+        assert sim.get_tile() == (32, 8, 32)
+        b = W.inflow_3d_block(40, 36, 30, 3, spacing=1.0 / 64.0)
+        sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        with torch.cuda.stream(torch.cuda.ExternalStream(sim.stream_handle())):
+            torch.cuda._sleep(int(1.0e9))
+        t0 = time.perf_counter()
+        tile = sim.get_tile()
+        waited = time.perf_counter() - t0
+        sim.synchronize()
+        slept = time.perf_counter() - t0
+        sim.run(1)
+        assert sim.get_tile() == tile
+    assert waited < 0.5 * slept, (waited, slept)
