@@ -77,6 +77,7 @@ void Ctx::release() {
     fused_items = 0;
     descs_valid = false;
     max_cells_fused = 0;
+    nsm = 0;
     d_hlist = nullptr;
     hlist_cap = 0;
     d_sim = nullptr;

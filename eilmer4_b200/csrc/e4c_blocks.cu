@@ -190,6 +190,7 @@ int Ctx::build_block(int ni, int nj, int nk, const double* vtx, const int* bc,
         v.W = v.U0 = v.dUdt0 = v.Fi = v.Fj = v.Fk = nullptr;
         v.cgeom = v.fgi = v.fgj = v.fgk = nullptr;
         max_cells_fused = std::max(max_cells_fused, int(nc));
+        load_tiles();
     } else {
         double* slab = static_cast<double*>(dalloc(nstate * sizeof(double)));
         if (!slab) return fail(E4C_ERR_CUDA, "cudaMalloc of block storage failed");
@@ -250,6 +251,7 @@ struct TileCost {
     int ti, tj;
     double plane, alone, start;
 };
+constexpr int kMostTiles = 5;
 static const TileCost kTiles64[] = {{32, 14, 10.4, 10.4, 8.0}, {32, 8, 6.5, 6.5, 7.0},
                                     {32, 4, 6.8, 4.5, 6.6},    {16, 16, 14.8, 9.5, 9.0},
                                     {16, 8, 16.4, 6.5, 16.0}};
@@ -263,14 +265,32 @@ static const TileCost kTiles32[] = {{32, 8, 5.3, 3.6, 7.5}, {32, 4, 4.7, 2.4, 10
 // 64x4 (the per-face kernel; 128^3 AUSMDV 1.12 and 1.83 ms/step against 1.07
 // with 32x8), FP32-flux 32x14 (256^3 HLLC 2.95 against 2.48 with 32x8).
 
-void Ctx::choose_tile() {
+static const TileCost* tile_costs(const e4c_config& cfg, int& n) {
+    static_assert(sizeof(kTiles64) <= kMostTiles * sizeof(TileCost) &&
+                  sizeof(kTiles32) <= kMostTiles * sizeof(TileCost), "room for the occupancies");
     const bool f32_form = cfg.precision == E4C_PREC_FP32_FLUX;
-    const TileCost* tiles = f32_form ? kTiles32 : kTiles64;
-    const int ntiles = f32_form ? int(sizeof(kTiles32) / sizeof(TileCost))
-                                : int(sizeof(kTiles64) / sizeof(TileCost));
-    static const int chunks[] = {4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64};
-    int nsm = 148, max_nk = 0;
+    n = f32_form ? int(sizeof(kTiles32) / sizeof(TileCost)) : int(sizeof(kTiles64) / sizeof(TileCost));
+    return f32_form ? kTiles32 : kTiles64;
+}
+
+// SMs of the device and resident CTAs of each shape's kernel per SM, asked for
+// once per context, when its first fused block is created: a kernel's first
+// query loads it, which waits for the device.
+void Ctx::load_tiles() {
+    if (nsm > 0) return;
+    int n;
+    const TileCost* tiles = tile_costs(cfg, n);
+    tile_per_sm.assign(kMostTiles, 0);
+    for (int q = 0; q < n; ++q) tile_per_sm[q] = fused_occupancy(tiles[q].ti, tiles[q].tj);
+    nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cfg.device);
+}
+
+void Ctx::choose_tile() {
+    int ntiles;
+    const TileCost* tiles = tile_costs(cfg, ntiles);
+    static const int chunks[] = {4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64};
+    int max_nk = 0;
     for (const BlockHost& b : blocks)
         if (b.fused) max_nk = std::max(max_nk, b.f.nk);
     if (max_nk == 0) return;
@@ -278,7 +298,7 @@ void Ctx::choose_tile() {
     std::vector<double> cost, busy;
     for (int q = 0; q < ntiles; ++q) {
         const TileCost& t = tiles[q];
-        const int per_sm = fused_occupancy(t.ti, t.tj);
+        const int per_sm = tile_per_sm[q];
         if (per_sm <= 0) continue;
         for (int kc : chunks) {
             cost.clear();
@@ -420,8 +440,6 @@ int Ctx::prepare_fused() {
         E4C_CUDA(cudaMemcpyAsync(d_item_order, order.data(), sizeof(int) * order.size(),
                                  cudaMemcpyHostToDevice, stream));
         E4C_CUDA(cudaStreamSynchronize(stream));
-        int nsm = 148;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, cfg.device);
         const int per_sm = fused_occupancy(tile_ti, tile_tj);
         if (per_sm <= 0) return fail(E4C_ERR_UNSUPPORTED, "fused tile shape does not fit on the device");
         long long g = (long long)nsm * per_sm;

@@ -129,6 +129,8 @@ struct Ctx {
     bool descs_valid = false;
     int tile_ti = 32, tile_tj = 8, tile_kc = 32;
     bool tile_auto = true;     // chosen by choose_tile, until e4c_set_tile or e4c_autotune
+    int nsm = 0;                      // SMs, and CTAs per SM of choose_tile's shapes
+    std::vector<int> tile_per_sm;     // (load_tiles)
     int fused_grid = 0;
     int max_cells_fused = 0;
     // device list of block handles for the dt reduction
@@ -147,6 +149,7 @@ struct Ctx {
     void dfree(void* p);
     int prepare_fused();
     void choose_tile();
+    void load_tiles();
     int fused_occupancy(int ti, int tj) const;
     int set_hlist(const std::vector<int>& hs);
     bool uses_all_fused(const std::vector<int>& hs) const;
