@@ -295,14 +295,13 @@ void Ctx::choose_tile() {
         if (b.fused) max_nk = std::max(max_nk, b.f.nk);
     if (max_nk == 0) return;
     double best = 1.0e300;
-    std::vector<double> cost, busy;
+    std::vector<std::pair<double, long long>> cost;   // cost of an item, items that have it
+    std::vector<double> busy;
     for (int q = 0; q < ntiles; ++q) {
         const TileCost& t = tiles[q];
         const int per_sm = tile_per_sm[q];
         if (per_sm <= 0) continue;
         for (int kc : chunks) {
-            cost.clear();
-            double total = 0.0, longest = 0.0;
             long long items = 0;
             for (const BlockHost& b : blocks)
                 if (b.fused)
@@ -313,35 +312,43 @@ void Ctx::choose_tile() {
                 ? std::min(1.0, std::max(0.0, double(items) / nsm - 1.0) / (per_sm - 1)) : 1.0;
             const double plane = t.alone + (t.plane - t.alone) * share;
             const long long slots = (long long)nsm * per_sm;
-            const bool exact = items <= 4096;
+            cost.clear();
+            double total = 0.0, longest = 0.0;
             for (const BlockHost& b : blocks) {
                 if (!b.fused) continue;
-                const int tiles_i = (b.f.ni + t.ti - 1) / t.ti;
-                for (int j0 = 0; j0 < b.f.nj; j0 += t.tj)
-                    for (int k0 = 0; k0 < b.f.nk; k0 += kc) {
+                // full and cut tiles (in j) times full and cut chunks
+                const long long tiles_i = (b.f.ni + t.ti - 1) / t.ti;
+                const int rows[2] = {t.tj, b.f.nj % t.tj}, planes[2] = {kc, b.f.nk % kc};
+                const int nrows[2] = {b.f.nj / t.tj, rows[1] > 0}, nplanes[2] = {b.f.nk / kc, planes[1] > 0};
+                for (int r = 0; r < 2; ++r)
+                    for (int p = 0; p < 2; ++p) {
+                        const long long n = tiles_i * nrows[r] * nplanes[p];
+                        if (n == 0) continue;
                         // rows beyond the block are skipped; the plane's fixed
                         // part (loads, edges, the barrier) stays
-                        const double rows = double(std::min(t.tj, b.f.nj - j0)) / t.tj;
-                        const double c = t.start + std::min(kc, b.f.nk - k0) * plane *
-                                                       (0.35 + 0.65 * rows);
-                        total += c * tiles_i;
+                        const double c =
+                            t.start + planes[p] * plane * (0.35 + 0.65 * rows[r] / t.tj);
+                        total += c * n;
                         longest = std::max(longest, c);
-                        if (exact) cost.insert(cost.end(), size_t(tiles_i), c);
+                        cost.push_back({c, n});
                     }
             }
+            // no schedule is shorter than this
+            const bool hopeless = std::max(longest, total / slots) >= best;
             double span = total / slots + longest;
-            if (exact) {
+            if (!hopeless && items <= 4096) {
                 // costliest first, each to the slot that is free first
-                std::sort(cost.begin(), cost.end(), std::greater<double>());
+                std::sort(cost.begin(), cost.end(), std::greater<>());
                 busy.assign(size_t(std::min<long long>(slots, items)), 0.0);
-                for (double c : cost) {
-                    std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-                    busy.back() += c;
-                    std::push_heap(busy.begin(), busy.end(), std::greater<double>());
-                }
+                for (const auto& c : cost)
+                    for (long long n = 0; n < c.second; ++n) {
+                        std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+                        busy.back() += c.first;
+                        std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+                    }
                 span = *std::max_element(busy.begin(), busy.end());
             }
-            if (span < best) {
+            if (!hopeless && span < best) {
                 best = span;
                 tile_ti = t.ti; tile_tj = t.tj; tile_kc = kc;
             }
