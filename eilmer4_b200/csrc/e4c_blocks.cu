@@ -243,7 +243,11 @@ int Ctx::fused_occupancy(int ti, int tj) const {
 // plane: microseconds per full plane with the SM's CTAs all resident; alone:
 // the same for a CTA that has the SM to itself; start: microseconds per item.
 // Measured with HLLC on the 256^3 block (chunks of 32, 16, 8 and 4 planes) and
-// on four joined 48x36x40 blocks; only their ratios matter.  Against the fixed
+// on four joined 48x36x40 blocks; only their ratios matter, and they serve the
+// other fluxes as well: over 25 layouts (27 K to 2.3 M cells) e4c_autotune finds
+// a step of 0.967 times the choice's on average with HLLC, 0.950 AUSMDV, 0.960
+// Hanel, 0.943 adaptive, 0.964 and 0.967 FP32-flux HLLC and AUSMDV (at best 0.69,
+// short chunks of a 251,856-cell block).  Against the fixed
 // 32x8 tile and 32-plane chunks (per stage, before -> chosen): the four
 // blocks 0.23 -> 0.11 ms, a 150x141x133 blast block 1.02 -> 0.93 ms, 64 uneven
 // blocks 2.04 -> 1.88 ms, 256^3 2.98 -> 2.80 ms.

@@ -413,10 +413,13 @@ int e4c_get_tile(int* ti, int* tj, int* kc);
  * the lengths (every length gives the same bits); they only set the speed. */
 int e4c_set_flux_runs(int i_faces, int jk_faces);
 
-/* Autotuner: time nsteps steps with every available tile shape and k-chunk
- * length on the current blocks, keep the fastest, and restore the flow state
- * and simulation clock exactly as they were before the trials.  Returns the
- * chosen shape and its milliseconds per step. */
+/* Autotuner: time nsteps steps with the shape in use (the automatic choice, or
+ * e4c_set_tile's), with every available shape at chunks of 16, 32, 64 and 128
+ * planes (and a shorter chunk in use), and with chunks around the best; keep the
+ * fastest (the shape in use, unless another is 1 % faster) until e4c_set_tile or
+ * e4c_init, and restore the flow state and simulation clock exactly as they
+ * were before the trials.  Returns the chosen shape and its milliseconds per
+ * step. */
 int e4c_autotune(int nsteps, int* ti, int* tj, int* kc, double* ms_per_step);
 
 /* Most blocks one e4c_dt_allow_noalloc call can reduce over. */

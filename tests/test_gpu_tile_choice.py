@@ -89,3 +89,36 @@ def test_choice_costs_little_host_time(e4lib):
             sim.get_tile()
             times.append(time.perf_counter() - t0)
     assert min(times) < 1.8e-3, times
+
+
+@pytest.mark.parametrize("sizes", [[(24, 24, 24)], [(64, 64, 64)], [(48, 36, 40)] * 4])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_flux"])
+def test_autotune_is_no_slower_than_the_choice(e4lib, sizes, precision):
+    """The tuner times the pair it finds in use beside its own list (whose chunks
+    start at 16 planes: alone it would end at three times the step on 24^3)."""
+    import torch
+
+    from eilmer4_b200.simcore import Simulation
+    with Simulation({"dimensions": 3, "flux_calculator": "ausmdv"}, precision=precision) as sim:
+        for n in sizes:
+            b = W.inflow_3d_block(*n, 3, spacing=1.0 / 64.0)
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        s = torch.cuda.ExternalStream(sim.stream_handle())
+
+        def ms_per_step():
+            sim.run(10)
+            best = 1.0e9
+            for _ in range(4):
+                e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                e[0].record(s)
+                sim.run(50)
+                e[1].record(s)
+                torch.cuda.synchronize()
+                best = min(best, e[0].elapsed_time(e[1]) / 50)
+            return best
+
+        untuned = ms_per_step()
+        tile, _ = sim.autotune(5)
+        assert sim.get_tile() == tile
+        tuned = ms_per_step()
+    assert tuned < 1.05 * untuned, (tile, tuned, untuned)
