@@ -130,7 +130,10 @@ __device__ __forceinline__ void load_frame(const double* fg, size_t npad, size_t
 // us/step with 5 -> 1 and with one division after another, curvilinear
 // 40x36x30 HLLC 117 -> 106 (106), 128^3 AUSMDV 1,653 -> 1,560 (1,658) and
 // adaptive 1,955 -> 1,808 (1,897), stretched 118x90x70 AUSMDV 468 -> 449 (500).
-constexpr int kFluxBatch = 3, kRowBatch = 1;
+// A launch whose CTAs all fit at 2 per SM loses no warps to the registers, and
+// there the shorter chain counts: k_flux_rows takes all 5 at once (100x2x2 tube,
+// 12 CTAs: 17 us a step in the flux kernels against 21).
+constexpr int kFluxBatch = 3, kRowBatch = 1, kRowBatchFew = 5, kRowFewCtas = 2 * 148;
 
 // rho, velocity and u of a face's two states from its four stencil cells (B:
 // scalars per batch of quotients)
@@ -467,7 +470,8 @@ constexpr int kRowThreads = 128;
 // parity) before the current face is computed, so their latency hides behind
 // its arithmetic.  Launched with kRowThreads threads per block.
 // MUTATE: the block's frames are general (b.Vrt holds the replayed bases).
-template <int NSP, int FLUX, int GAS, bool MUTATE>
+// BATCH: kRowBatch, or kRowBatchFew for at most kRowFewCtas CTAs.
+template <int NSP, int FLUX, int GAS, bool MUTATE, int BATCH>
 __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const SimDev* sim,
                                                           FluxOpts o, int3 runs) {
     static_assert(NSP == 1, "the row walk serves ideal-gas blocks");
@@ -602,9 +606,9 @@ __global__ void __launch_bounds__(kRowThreads) k_flux_rows(BlockView b, const Si
             {
                 L2R2<double> r;
                 r.prepare(wl[0], wl[1], wl[2], wl[3]);
-                interp_face<NSP, kRowBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                interp_face<NSP, BATCH>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                 if (NSP > 1) {
-                    interp_massf<NSP, kRowBatch>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
+                    interp_massf<NSP, BATCH>(r, o.limiter, o.clip, sL1, sL0, sR0, sR1, Lf, Rt);
                     if (!scale_mass_fractions<double, NSP>(Lf.massf))
                         for (int q = 0; q < NSP; ++q) Lf.massf[q] = sL0.massf[q];
                     if (!scale_mass_fractions<double, NSP>(Rt.massf))

@@ -838,6 +838,24 @@ int3 flux_row_runs(const BlockView& b, const FluxOpts& o) {
     return make_int3(r[0], r[1], r[2]);
 }
 
+template <bool MUTATE, int FLUX>
+static void launch_flux_rows_of(const BlockView& b, const SimDev* sim, const FluxOpts& o,
+                                const int3& runs, int g, cudaStream_t s) {
+    if (g <= kRowFewCtas)
+        launch_pdl(k_flux_rows<1, FLUX, 0, MUTATE, kRowBatchFew>, g, kRowThreads, 0, s, b, sim, o, runs);
+    else
+        launch_pdl(k_flux_rows<1, FLUX, 0, MUTATE, kRowBatch>, g, kRowThreads, 0, s, b, sim, o, runs);
+}
+
+template <bool MUTATE>
+static void launch_flux_rows(const BlockView& b, const SimDev* sim, const FluxOpts& o,
+                             const int3& runs, int g, cudaStream_t s) {
+    if (o.flux == 1) launch_flux_rows_of<MUTATE, 1>(b, sim, o, runs, g, s);
+    else if (o.flux == 2) launch_flux_rows_of<MUTATE, 2>(b, sim, o, runs, g, s);
+    else if (o.flux == 3) launch_flux_rows_of<MUTATE, 3>(b, sim, o, runs, g, s);
+    else launch_flux_rows_of<MUTATE, 0>(b, sim, o, runs, g, s);
+}
+
 void launch_flux(const BlockView& b, const SimDev* sim, const FluxOpts& o, int dir,
                  cudaStream_t s) {
     if (dir < 0 && o.order2 && o.local_frame && b.dim == 3 && b.nsp == 1) {
@@ -849,19 +867,9 @@ void launch_flux(const BlockView& b, const SimDev* sim, const FluxOpts& o, int d
         const int3 runs = flux_row_runs(b, o);
         const int r[3] = {runs.x, runs.y, runs.z};
         const long long n = row_threads(b, r);
-        const int T = kRowThreads;
-        const int g = grid_for(n, T);
-        if (b.Vrt) {
-            if (o.flux == 1) launch_pdl(k_flux_rows<1, 1, 0, true>, g, T, 0, s, b, sim, o, runs);
-            else if (o.flux == 2) launch_pdl(k_flux_rows<1, 2, 0, true>, g, T, 0, s, b, sim, o, runs);
-            else if (o.flux == 3) launch_pdl(k_flux_rows<1, 3, 0, true>, g, T, 0, s, b, sim, o, runs);
-            else launch_pdl(k_flux_rows<1, 0, 0, true>, g, T, 0, s, b, sim, o, runs);
-        } else {
-            if (o.flux == 1) launch_pdl(k_flux_rows<1, 1, 0, false>, g, T, 0, s, b, sim, o, runs);
-            else if (o.flux == 2) launch_pdl(k_flux_rows<1, 2, 0, false>, g, T, 0, s, b, sim, o, runs);
-            else if (o.flux == 3) launch_pdl(k_flux_rows<1, 3, 0, false>, g, T, 0, s, b, sim, o, runs);
-            else launch_pdl(k_flux_rows<1, 0, 0, false>, g, T, 0, s, b, sim, o, runs);
-        }
+        const int g = grid_for(n, kRowThreads);
+        if (b.Vrt) launch_flux_rows<true>(b, sim, o, runs, g, s);
+        else launch_flux_rows<false>(b, sim, o, runs, g, s);
         return;
     }
     long long n = 0;

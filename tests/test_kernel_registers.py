@@ -16,7 +16,7 @@ SOURCE = """
 #include "e4c_internal.h"
 #include "e4c_cells.cuh"
 namespace e4c {
-#define ROWS(F, M) template __global__ void k_flux_rows<1, F, 0, M>(BlockView, const SimDev*, FluxOpts, int3);
+#define ROWS(F, M) template __global__ void k_flux_rows<1, F, 0, M, kRowBatch>(BlockView, const SimDev*, FluxOpts, int3);
 ROWS(0, false) ROWS(1, true) ROWS(3, true)
 template __global__ void k_flux<1, 1, 0>(BlockView, const SimDev*, FluxOpts, int);
 template __global__ void k_flux<1, 3, 0>(BlockView, const SimDev*, FluxOpts, int);
