@@ -340,7 +340,7 @@ def test_conserved_upload_rejects_bad_mass_and_the_mixture(e4lib):
         assert err.value.code == _lib.E4C_ERR_UNSUPPORTED
 
 
-@pytest.mark.parametrize("tile", [(32, 4, 7), (32, 8, 16), (32, 16, 64), (16, 16, 16)])
+@pytest.mark.parametrize("tile", [(32, 4, 7), (32, 8, 16), (32, 16, 64), (32, 14, 9), (16, 16, 16)])
 @pytest.mark.parametrize("case", ["inflow", "walls"])
 def test_fp32_flux_tile_shapes_error_vs_fp64(oracle, e4lib, tile, case):
     """The FP32-flux form with each kernel and tile shape it runs: 32-wide

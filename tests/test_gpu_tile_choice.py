@@ -38,6 +38,25 @@ def test_chosen_tile(oracle, e4lib, sizes):
         assert sim.get_tile() == (ti, tj, kc)
 
 
+def test_choices_of_several_layouts(oracle, e4lib):
+    """Layouts for which the model takes different shapes (a long narrow block,
+    cubes, a flat one), each with the oracle's bits."""
+    from eilmer4_b200.simcore import Simulation
+    chosen = []
+    for n in [(24, 24, 24), (7, 83, 120), (96, 96, 96), (120, 112, 40)]:
+        b = W.inflow_3d_block(*n, 3, spacing=1.0 / 64.0)
+        ref = oracle.OracleSim(oracle.default_config(dimensions=3, flux_calculator=FLUX["hllc"],
+                                                     n_threads=0))
+        ref.set_flow(ref.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+        with Simulation({"dimensions": 3, "flux_calculator": "hllc"}) as sim:
+            sim.upload(sim.add_block(b.ni, b.nj, b.nk, b.vtx, b.bc, b.inflow), b.prim)
+            chosen.append(sim.get_tile())
+            assert ref.run(4) == 0
+            sim.run(4)
+            assert_same(sim.download(0)[1], ref.get_flow(0)[1], f"{n}, tile {chosen[-1]}")
+    assert len({c[:2] for c in chosen}) >= 3, chosen
+
+
 @pytest.mark.parametrize("sizes", [[(48, 96, 96), (48, 96, 96)], [(96, 96, 96)], [(112, 112, 114)],
                                    [(40, 88, 91)], [(16, 64, 48)] * 9])
 def test_fp32_choice_keeps_the_edge_warp_kernel(e4lib, sizes):
