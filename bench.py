@@ -66,21 +66,19 @@ BYTES_PER_CELL_UPDATE = {"fp64": 360.0, "fp32_flux": 280.0}
 # massf x5, T, p, u, a, dt_chem and rho*massf x5 (doubles)
 BYTES_PER_REACTING_CELL = 8.0 * (9 + 15)
 # DRAM bytes per launch of the fused stage kernel (dram__bytes_read.sum +
-# dram__bytes_write.sum, mean of the stage-1 and stage-2 launches) from ncu
-# captures, keyed by (precision, kernel class), for the autotuner's picks:
-# FP64 (32x16 tile, 32-plane k-chunks) captured on the 128^3 block and scaled
-# to 256^3 by the cell count (the kernel's traffic grows with the cells it
-# processes); FP32-flux (the 32x8 tile of the edge-warp kernel, 32-plane
-# k-chunks) captured on the 256^3 block itself.  Algorithmic bytes per launch
-# at 256^3: 3020 MB (FP64), 2349 MB (FP32-flux).
-TRAFFIC = {("fp64", "stage"): 2758515712, ("fp32_flux", "stage"): 2418098712}
-# FP64 arithmetic per cell-update of the fused stage kernel (both stages),
-# keyed by (precision, flux): DADD + DMUL + 2 x DFMA thread instructions per
-# cycle times cycles, from the ncu capture of the 128^3 block with the 32x16
-# tile (the count per cell does not depend on the block size for a tile
-# shape).  Compiled without FMA contraction, the kernel's ceiling is half the
-# FP64 peak (64 DFMA per SM per cycle, 2 FLOP each).
-FP64_FLOP_PER_CELL_UPDATE = {("fp64", "hllc"): 2430.0}
+# dram__bytes_write.sum, mean of the stage-1 and stage-2 launches) at 256^3 from
+# one-pass ncu captures of that block, keyed by (precision, kernel class, flux),
+# with the autotuner's picks: FP64 32x14 and 40-plane chunks, FP32-flux 32x8 and
+# 48.  Algorithmic bytes per launch: 3020 MB (FP64), 2349 MB (FP32-flux).
+TRAFFIC = {("fp64", "stage", "hllc"): 3156420000, ("fp32_flux", "stage", "hllc"): 2387944000}
+# FP64 arithmetic per cell-update of the fused stage kernel (both stages), keyed
+# by (precision, flux): DADD + DMUL + 2 x DFMA thread instructions from the ncu
+# capture of the 128^3 block with the 32x14 tile, and the instructions they are
+# (575 DADD, 763 DMUL, 396 DFMA: the quotients' steps are fused, everything else
+# rounds as the reference does).  The peak counts two FLOP per instruction, so
+# FLOP / (2 x instructions) of it is the mix's ceiling.
+FP64_FLOP_PER_CELL_UPDATE = {("fp64", "hllc"): 2130.0}
+FP64_INST_PER_CELL_UPDATE = {("fp64", "hllc"): 1734.0}
 
 
 def oracle_flux(O, flux):
@@ -429,7 +427,7 @@ def euler_case(args, precision, local_rank, dist, world, headline, flux=None):
                  "autotuned": not (args.no_autotune or args.tile)},
         "roofline": {"bound": "hbm", "kernel": cls, "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind,
-                     "traffic": TRAFFIC.get((precision, cls)),
+                     "traffic": TRAFFIC.get((precision, cls, flux)),
                      "step_achieved": step_achieved, "step_frac": step_achieved / hbm,
                      "bytes_per_cell_update": bpc},
         "profile_ms": {k: round(v[0] / args.profile_steps, 4) for k, v in prof.items()},
@@ -445,7 +443,9 @@ def euler_case(args, precision, local_rank, dist, world, headline, flux=None):
         ach_tf = achieved * fpc / bpc / 1e3
         res["fp64_roofline"] = {"bound": "fp64", "kernel": cls, "achieved": ach_tf,
                                 "peak": peak_tf, "unit": "TFLOP/s", "frac": ach_tf / peak_tf,
-                                "flop_per_cell_update": fpc, "no_fma_ceiling_frac": 0.5,
+                                "flop_per_cell_update": fpc,
+                                "mix_ceiling_frac":
+                                    fpc / (2.0 * FP64_INST_PER_CELL_UPDATE[(precision, flux)]),
                                 "peak_kind": "64 DFMA per SM per cycle at the sampled SM clock"}
     if clk is not None:
         res["clocks"] = clk
