@@ -9,7 +9,8 @@
 // per direction and computes its west, south and top faces.
 //
 // What bounds it: FP64 instruction issue and the latency of its dependency
-// chains (the reference's rounding allows no fused multiply-adds), not HBM.
+// chains (the reference's rounding allows no fused multiply-adds outside the
+// quotients), not HBM.
 // So the split is chosen for operations and for warps in flight:
 //   * per-cell reconstruction: one set of differences, limiter values and MUSCL
 //     values per cell and direction (the per-face form computes the
@@ -26,11 +27,11 @@
 // 16 warps at 128 registers: fewer registers spill, more of them cost warps
 // (20 warps at 96 registers measured 6.7 ms/step where 16 took 5.8).
 // Measured on the 256^3 block, HLLC, per step: 7.53 ms for the per-face kernel
-// with the 32x8 tile and 32-plane chunks, 6.57 with its best tile (32x16);
-// 5.98 here with 32x8, 5.59 with 32x14.  128^3, 32x14 (ncu): 2,170
-// instructions per warp and plane, 40 % of them FP64, 0.46 issued per cycle
-// and scheduler, stalls led by the FP64 chains (2.3 of 8.6 cycles) and the
-// barrier (1.6).
+// with the 32x8 tile and 32-plane chunks, 6.57 with its best tile (32x16; both
+// before the batched quotients, 6.47 with them); 5.99 here with 32x8, 5.57 with
+// 32x14, 5.46 with that and 40-plane chunks.  128^3, 32x14 (ncu): 31 % of the
+// instructions are FP64, 0.47 issued per cycle and scheduler, stalls led by the
+// FP64 chains (2.2 cycles per instruction issued) and the barrier (1.2).
 //
 // The arithmetic is that of the per-face kernel (e4c_fused.cuh), operation for
 // operation, so results are the same bits.  On a uniform grid the left state of

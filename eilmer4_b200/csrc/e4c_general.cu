@@ -649,8 +649,9 @@ __device__ __forceinline__ void end_of_step(SimDev* sim) {
 
 // The stage's invalid cells (simcore.d:2480-2493), its count taken over and
 // cleared for the next stage; on the last stage of a step without chemistry
-// the step's end as well.  (A launch of its own for each cost a small block
-// about a quarter of its step: 11 kernels a step -> 8.)
+// the step's end as well.  (With a launch of its own for each, 11 kernels a step
+// for 8, and no overlap of launches, the 100x2x2 tube took 49 us a step against
+// 41 and the 256x64 block 56 against 53.)
 __global__ void k_stage_check(SimDev* sim, int max_invalid_cells, int end_step) {
     pdl_wait();
     const int bad = sim->bad_acc;
