@@ -246,8 +246,8 @@ int Ctx::fused_occupancy(int ti, int tj) const {
 // on four joined 48x36x40 blocks; only their ratios matter, and they serve the
 // other fluxes as well: over 25 layouts (27 K to 2.3 M cells) e4c_autotune finds
 // a step of 0.967 times the choice's on average with HLLC, 0.950 AUSMDV, 0.960
-// Hanel, 0.943 adaptive, 0.964 and 0.967 FP32-flux HLLC and AUSMDV (at best 0.69,
-// short chunks of a 251,856-cell block).  Against the fixed
+// Hanel, 0.943 adaptive, 0.964 and 0.967 FP32-flux HLLC and AUSMDV (at best 0.69:
+// 251,856 cells, adaptive, 32x16 for 32x14, both with 5-plane chunks).  Against the fixed
 // 32x8 tile and 32-plane chunks (per stage, before -> chosen): the four
 // blocks 0.23 -> 0.11 ms, a 150x141x133 blast block 1.02 -> 0.93 ms, 64 uneven
 // blocks 2.04 -> 1.88 ms, 256^3 2.98 -> 2.80 ms.
@@ -265,9 +265,10 @@ static const TileCost kTiles64[] = {{32, 14, 10.4, 10.4, 8.0}, {32, 8, 6.5, 6.5,
 // a block's results depended on which kernel the other blocks' sizes selected.
 static const TileCost kTiles32[] = {{32, 8, 5.3, 3.6, 7.5}, {32, 4, 4.7, 2.4, 10.0},
                                     {32, 16, 5.7, 5.7, 9.0}};
-// Not among the choices, slower wherever they were measured: FP64 32x16 and
-// 64x4 (the per-face kernel; 128^3 AUSMDV 1.12 and 1.83 ms/step against 1.07
-// with 32x8), FP32-flux 32x14 (256^3 HLLC 2.95 against 2.48 with 32x8).
+// Not among the choices: FP64 32x16 and 64x4, the per-face kernel (128^3 AUSMDV
+// 1.12 and 1.83 ms/step against 1.07 with 32x8; on a few layouts e4c_autotune
+// does find them the fastest), and FP32-flux 32x14 (256^3 HLLC 2.95 against 2.48
+// with 32x8).
 
 static const TileCost* tile_costs(const e4c_config& cfg, int& n) {
     static_assert(sizeof(kTiles64) <= kMostTiles * sizeof(TileCost) &&
